@@ -7,11 +7,12 @@
 // backward, as the reference does, allocates through torch's caching allocator and makes one C call per direction.
 //
 // linear() and conv2d() answer None for whatever it does not cover (other transform schemes, the logarithmic quantiser, token
-// bases above 64, other dtypes or devices, arguments that are in error); the caller then takes the Python Function,
+// bases above 64, other dtypes or devices, autocast, arguments that are in error); the caller then takes the Python Function,
 // which covers or refuses it.  A configuration that leaves the covered set between forward and backward
 // goes to that Function's backward too.
 #include <torch/extension.h>
 
+#include <ATen/autocast_mode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
@@ -342,6 +343,7 @@ struct HotConvBackward : public Node {
 // The part of a layer's configuration that forward fixes; false: not covered (a Python error may be pending).
 // a: x, w, bias or None, order_o, order_l, selection, name
 bool forward_config(PyObject* const* a, hot_linear_cfg_t& c, bool& preset) {
+  if (at::autocast::is_autocast_enabled(at::kCUDA)) return false;  // the product would come in autocast's type, not the tensors'
   if (!THPVariable_Check(a[0]) || !THPVariable_Check(a[1]) || !PyList_Check(a[5])) return false;
   const Tensor &x = THPVariable_Unpack(a[0]), &w = THPVariable_Unpack(a[1]);
   const int dt = dtype_code(x.scalar_type());
@@ -423,7 +425,7 @@ PyObject* linear_impl(PyObject* const* a) {
     const bool fused = bias.defined() && l.cfg.dtype == HOT_BF16;
     y = fused ? at::linear(x, w, bias) : at::linear(x, w);
     if (bias.defined() && !fused) {
-      if (y.is_contiguous() && bias.is_contiguous() && bias.numel() == l.O && bias.device() == y.device())
+      if (y.scalar_type() == at::kFloat && y.is_contiguous() && bias.is_contiguous() && bias.numel() == l.O && bias.device() == y.device())
         check(hot_add_bias((float*)y.data_ptr(), (const float*)bias.data_ptr(), y.numel() / l.O, l.O, current_stream()), "hot_add_bias");
       else y.add_(bias);
     }
@@ -475,6 +477,7 @@ PyObject* conv2d_impl(PyObject* const* a) {
     if (data_grads) compress(l, cols, node->s);
     else if (node) node->s.layer = l;
     const Tensor rows = at::linear(cols, w.view({l.O, l.I}));
+    TORCH_CHECK(rows.scalar_type() == x.scalar_type() && rows.is_contiguous(), "HQ_Conv2d: the product came back in another type or layout");
     y = at::empty({v.B, l.O, oh, ow}, x.options());
     check(hot_transpose(v.dtype, v.B, positions, l.O, rows.data_ptr(), bias.defined() ? bias.data_ptr() : nullptr, y.data_ptr(), current_stream()),
           "hot_transpose");
