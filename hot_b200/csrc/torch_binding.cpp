@@ -260,13 +260,18 @@ struct Saved {
       shape.back() = l.I;
       gx = at::empty(shape, go.options());
     }
-    if (need_w) gw = at::empty({l.O, l.I}, go.options());
+    // the product summed over samples is stored through a tensor map, whose rows begin at multiples of 16 bytes
+    int64_t ldgw = l.I;
+    const int64_t per16 = 16 / (int64_t)go.element_size();
+    if (l.batch) ldgw = (ldgw + per16 - 1) / per16 * per16;
+    if (need_w) gw = at::empty({l.O, ldgw}, go.options());
     // the bias gradient comes from the quantisers' own pass over grad_out (they take channels in pairs)
     if (need_b) gb = l.O % 2 == 0 ? at::empty({l.O}, go.options()) : go.reshape({-1, l.O}).sum(0);
     check(hot_layer_backward(&l, go.data_ptr(), w2.data_ptr(), w2.stride(0), x_q_t.data_ptr(), (const float*)scale_x.data_ptr(),
-                             need_x ? gx.data_ptr() : nullptr, l.I, need_w ? gw.data_ptr() : nullptr, l.I, need_b && l.O % 2 == 0 ? gb.data_ptr() : nullptr,
+                             need_x ? gx.data_ptr() : nullptr, l.I, need_w ? gw.data_ptr() : nullptr, ldgw, need_b && l.O % 2 == 0 ? gb.data_ptr() : nullptr,
                              ws.data_ptr(), ws_bytes, nullptr, current_stream()),
           "hot_layer_backward");
+    if (need_w && ldgw != l.I) gw = gw.narrow(1, 0, l.I);
   }
 };
 
@@ -330,7 +335,7 @@ struct HotConvBackward : public Node {
     Tensor gb;
     s.backward(rows, w.view({s.layer.O, s.layer.I}), need_x, need_w, need_b, gcols, out[1], gb);
     if (need_b) out[2] = gb;
-    if (need_w) out[1] = out[1].view(w.sizes());
+    if (need_w) out[1] = out[1].reshape(w.sizes());  // (a copy where its rows are padded)
     if (need_x) {
       gcols = gcols.contiguous();
       out[0] = at::empty({conv.B, conv.C, conv.H, conv.W}, go.options());
