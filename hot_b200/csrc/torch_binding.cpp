@@ -210,7 +210,6 @@ struct Saved {
   Tensor x_q_t, scale_x;
   hot_layer_t layer = {};
   PyObject* name = nullptr;
-  bool freed = false;
 
   ~Saved() {
     if (name && Py_IsInitialized()) {
@@ -222,7 +221,6 @@ struct Saved {
     w.reset_data();
     x_q_t.reset();
     scale_x.reset();
-    freed = true;
   }
   // (batch, order_o, order_l, selection, q_x bits, q_x packed): what the Python backward needs to know of the forward
   Ref describe() const {
@@ -234,10 +232,6 @@ struct Saved {
   // go: contiguous, w2: the weight as [O, I], both of one dtype; gx comes in the shape of go with I in place of O
   void backward(const Tensor& go, const Tensor& w2, bool need_x, bool need_w, bool need_b, Tensor& gx, Tensor& gw, Tensor& gb) const {
     hot_layer_t l = layer;
-    if (!need_x && !need_w) {
-      if (need_b) gb = go.reshape({-1, l.O}).sum(0);
-      return;
-    }
     {
       pybind11::gil_scoped_acquire gil;
       if (!backward_quantisers(name, l.cfg)) {
@@ -282,15 +276,18 @@ struct HotLinearBackward : public Node {
   void release_variables() override { s.release(); }
 
   variable_list apply(variable_list&& grads) override {
-    TORCH_CHECK(!s.freed, torch::autograd::ERR_BACKWARD_TWICE);
     variable_list out(has_bias ? 3 : 2);
     if (!grads[0].defined()) return out;
     at::NoGradGuard no_grad;
-    const Tensor w = s.w.unpack(shared_from_this()).detach();
-    c10::cuda::CUDAGuard guard(w.device());
     Tensor go = grads[0];
     const bool need_x = task_should_compute_output(0), need_w = task_should_compute_output(1);
     bool need_b = has_bias && task_should_compute_output(2);
+    if (!need_x && !need_w) {  // (needs nothing of what forward saved, and forward saved nothing where only the bias learns)
+      if (need_b) out[2] = go.reshape({-1, go.size(-1)}).sum(0);
+      return out;
+    }
+    const Tensor w = s.w.unpack(shared_from_this()).detach();
+    c10::cuda::CUDAGuard guard(w.device());
     if (need_b && go.scalar_type() != w.scalar_type()) {  // (the sum is taken in the type the gradient came in)
       out[2] = go.reshape({-1, go.size(-1)}).sum(0);
       need_b = false;
@@ -313,20 +310,22 @@ struct HotConvBackward : public Node {
   void release_variables() override { s.release(); }
 
   variable_list apply(variable_list&& grads) override {
-    TORCH_CHECK(!s.freed, torch::autograd::ERR_BACKWARD_TWICE);
     variable_list out(has_bias ? 3 : 2);
     if (!grads[0].defined()) return out;
     at::NoGradGuard no_grad;
-    const Tensor w = s.w.unpack(shared_from_this()).detach();
-    c10::cuda::CUDAGuard guard(w.device());
     Tensor go = grads[0];
     const bool need_x = task_should_compute_output(0), need_w = task_should_compute_output(1);
     bool need_b = has_bias && task_should_compute_output(2);
-    if (need_b && ((!need_x && !need_w) || go.scalar_type() != w.scalar_type())) {
+    if (!need_x && !need_w) {
+      if (need_b) out[2] = go.sum({0, 2, 3});
+      return out;
+    }
+    const Tensor w = s.w.unpack(shared_from_this()).detach();
+    c10::cuda::CUDAGuard guard(w.device());
+    if (need_b && go.scalar_type() != w.scalar_type()) {
       out[2] = go.sum({0, 2, 3});
       need_b = false;
     }
-    if (!need_x && !need_w) return out;
     go = go.contiguous();
     if (go.scalar_type() != w.scalar_type()) go = go.to(w.scalar_type());
     const Tensor rows = at::empty({conv.B, positions, s.layer.O}, go.options());
@@ -394,7 +393,7 @@ bool wants_grad(const Tensor& t) { return t.defined() && at::GradMode::is_enable
 template <typename NodeT>
 void attach(const std::shared_ptr<NodeT>& node, Tensor& y, const Tensor& x, const Tensor& w, const Tensor& bias, PyObject* name) {
   node->set_next_edges(bias.defined() ? torch::autograd::collect_next_edges(x, w, bias) : torch::autograd::collect_next_edges(x, w));
-  node->s.w = SavedVariable(w, false);
+  if (node->s.x_q_t.defined()) node->s.w = SavedVariable(w, false);  // (else only the bias learns: nothing is needed of forward)
   node->s.name = Py_NewRef(name);
   node->has_bias = bias.defined();
   torch::autograd::set_history(y, node);
@@ -480,7 +479,6 @@ PyObject* conv2d_impl(PyObject* const* a) {
     const Tensor xc = x.contiguous(), cols = at::empty({v.B, positions, l.I}, x.options());
     check(hot_im2col(&v, xc.data_ptr(), cols.data_ptr(), current_stream()), "hot_im2col");
     if (data_grads) compress(l, cols, node->s);
-    else if (node) node->s.layer = l;
     const Tensor rows = at::linear(cols, w.view({l.O, l.I}));
     TORCH_CHECK(rows.scalar_type() == x.scalar_type() && rows.is_contiguous(), "HQ_Conv2d: the product came back in another type or layout");
     y = at::empty({v.B, l.O, oh, ow}, x.options());
