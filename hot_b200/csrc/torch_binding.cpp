@@ -204,10 +204,10 @@ hot_stream_t current_stream() { return (hot_stream_t)c10::cuda::getCurrentCUDASt
 Tensor bytes(int64_t n, const Tensor& like) { return at::empty({n}, like.options().dtype(at::kByte)); }
 
 // ---- the autograd nodes --------------------------------------------------------------------------
-// What a layer keeps from forward to backward, and its two gradients from the gradient of its output rows.
+// What a layer keeps from forward to backward, and its two gradients from the gradient of its output rows.  The tensors are
+// saved variables, in the order of FLinearQ: saved-tensor hooks (offloading, checkpoints) see each of them.
 struct Saved {
-  SavedVariable w;  // [O, I], or a convolution's [O, C, kh, kw]
-  Tensor x_q_t, scale_x;
+  SavedVariable x_q_t, w, scale_x;  // w: [O, I], or a convolution's [O, C, kh, kw]
   hot_layer_t layer = {};
   PyObject* name = nullptr;
 
@@ -218,9 +218,9 @@ struct Saved {
     }
   }
   void release() {
+    x_q_t.reset_data();
     w.reset_data();
-    x_q_t.reset();
-    scale_x.reset();
+    scale_x.reset_data();
   }
   // (batch, order_o, order_l, selection, q_x bits, q_x packed): what the Python backward needs to know of the forward
   Ref describe() const {
@@ -230,13 +230,15 @@ struct Saved {
     return Ref(Py_BuildValue("(LiiNii)", (long long)layer.batch, c.order_o, c.order_l, sel, c.q_x.bits, c.q_x.storage == HOT_STORE_INT4));
   }
   // go: contiguous, w2: the weight as [O, I], both of one dtype; gx comes in the shape of go with I in place of O
-  void backward(const Tensor& go, const Tensor& w2, bool need_x, bool need_w, bool need_b, Tensor& gx, Tensor& gw, Tensor& gb) const {
+  void backward(const std::shared_ptr<Node>& node, const Tensor& go, const Tensor& w2, bool need_x, bool need_w, bool need_b, Tensor& gx,
+                Tensor& gw, Tensor& gb) const {
+    const Tensor codes = x_q_t.unpack(node), scale = scale_x.unpack(node);
     hot_layer_t l = layer;
     {
       pybind11::gil_scoped_acquire gil;
       if (!backward_quantisers(name, l.cfg)) {
         Ref r(PyObject_CallMethodObjArgs(g_qm, N.fallback, Ref(THPVariable_Wrap(go)).p, Ref(THPVariable_Wrap(w2)).p,
-                                         Ref(THPVariable_Wrap(x_q_t)).p, Ref(THPVariable_Wrap(scale_x)).p, describe().p, name,
+                                         Ref(THPVariable_Wrap(codes)).p, Ref(THPVariable_Wrap(scale)).p, describe().p, name,
                                          need_x ? Py_True : Py_False, need_w ? Py_True : Py_False, nullptr));
         if (!r) throw_python();
         PyObject *px = PyTuple_GetItem(r.p, 0), *pw = PyTuple_GetItem(r.p, 1);
@@ -261,7 +263,7 @@ struct Saved {
     if (need_w) gw = at::empty({l.O, ldgw}, go.options());
     // the bias gradient comes from the quantisers' own pass over grad_out (they take channels in pairs)
     if (need_b) gb = l.O % 2 == 0 ? at::empty({l.O}, go.options()) : go.reshape({-1, l.O}).sum(0);
-    check(hot_layer_backward(&l, go.data_ptr(), w2.data_ptr(), w2.stride(0), x_q_t.data_ptr(), (const float*)scale_x.data_ptr(),
+    check(hot_layer_backward(&l, go.data_ptr(), w2.data_ptr(), w2.stride(0), codes.data_ptr(), (const float*)scale.data_ptr(),
                              need_x ? gx.data_ptr() : nullptr, l.I, need_w ? gw.data_ptr() : nullptr, ldgw, need_b && l.O % 2 == 0 ? gb.data_ptr() : nullptr,
                              ws.data_ptr(), ws_bytes, nullptr, current_stream()),
           "hot_layer_backward");
@@ -295,7 +297,7 @@ struct HotLinearBackward : public Node {
     go = go.contiguous();
     if (go.scalar_type() != w.scalar_type()) go = go.to(w.scalar_type());
     Tensor gb;
-    s.backward(go, w, need_x, need_w, need_b, out[0], out[1], gb);
+    s.backward(shared_from_this(), go, w, need_x, need_w, need_b, out[0], out[1], gb);
     if (need_b) out[2] = gb;
     return out;
   }
@@ -332,7 +334,7 @@ struct HotConvBackward : public Node {
     check(hot_transpose(conv.dtype, conv.B, s.layer.O, positions, go.data_ptr(), nullptr, rows.data_ptr(), current_stream()), "hot_transpose");
     Tensor gcols;
     Tensor gb;
-    s.backward(rows, w.view({s.layer.O, s.layer.I}), need_x, need_w, need_b, gcols, out[1], gb);
+    s.backward(shared_from_this(), rows, w.view({s.layer.O, s.layer.I}), need_x, need_w, need_b, gcols, out[1], gb);
     if (need_b) out[2] = gb;
     if (need_w) out[1] = out[1].reshape(w.sizes());  // (a copy where its rows are padded)
     if (need_x) {
@@ -376,24 +378,34 @@ bool forward_config(PyObject* const* a, hot_linear_cfg_t& c, bool& preset) {
   return true;
 }
 
-// Takes the Philox offset of the activation buffer and makes it from the rows of x (contiguous).
-void compress(hot_layer_t& l, const Tensor& x, Saved& s) {
-  s.x_q_t = at::empty({l.I, hot_layer_buffer_pitch(&l)}, x.options().dtype(at::kByte));
-  s.scale_x = at::empty({std::max<int64_t>(l.batch, 1)}, x.options().dtype(at::kFloat));
+// The activation buffer, made from the rows of x (contiguous).
+struct Buffer {
+  Tensor codes, scale;
+};
+Buffer compress(const hot_layer_t& l, const Tensor& x) {
+  Buffer b;
+  b.codes = at::empty({l.I, hot_layer_buffer_pitch(&l)}, x.options().dtype(at::kByte));
+  b.scale = at::empty({std::max<int64_t>(l.batch, 1)}, x.options().dtype(at::kFloat));
   const size_t ws_bytes = hot_layer_compress_workspace_bytes(&l);
   if (ws_bytes == 0) fail(HOT_ERR_UNSUPPORTED, "hot_layer_compress");
   const Tensor ws = bytes((int64_t)ws_bytes, x);
-  check(hot_layer_compress(&l, x.data_ptr(), l.I, s.x_q_t.data_ptr(), (float*)s.scale_x.data_ptr(), ws.data_ptr(), ws_bytes, current_stream()),
+  check(hot_layer_compress(&l, x.data_ptr(), l.I, b.codes.data_ptr(), (float*)b.scale.data_ptr(), ws.data_ptr(), ws_bytes, current_stream()),
         "hot_layer_compress");
-  s.layer = l;
+  return b;
 }
 
 bool wants_grad(const Tensor& t) { return t.defined() && at::GradMode::is_enabled() && t.requires_grad(); }
 
 template <typename NodeT>
-void attach(const std::shared_ptr<NodeT>& node, Tensor& y, const Tensor& x, const Tensor& w, const Tensor& bias, PyObject* name) {
+void attach(const std::shared_ptr<NodeT>& node, Tensor& y, const Tensor& x, const Tensor& w, const Tensor& bias, const hot_layer_t& layer,
+            const Buffer& buffer, PyObject* name) {
   node->set_next_edges(bias.defined() ? torch::autograd::collect_next_edges(x, w, bias) : torch::autograd::collect_next_edges(x, w));
-  if (node->s.x_q_t.defined()) node->s.w = SavedVariable(w, false);  // (else only the bias learns: nothing is needed of forward)
+  if (buffer.codes.defined()) {  // (else only the bias learns: nothing is needed of forward)
+    node->s.x_q_t = SavedVariable(buffer.codes, false);
+    node->s.w = SavedVariable(w, false);
+    node->s.scale_x = SavedVariable(buffer.scale, false);
+  }
+  node->s.layer = layer;
   node->s.name = Py_NewRef(name);
   node->has_bias = bias.defined();
   torch::autograd::set_history(y, node);
@@ -416,6 +428,7 @@ PyObject* linear_impl(PyObject* const* a) {
   if (!per_sample && l.cfg.q_x.bits <= 4) l.cfg.q_x.storage = HOT_STORE_INT4;  // the saved buffer of the plain layout stays packed
   l.cfg.q_x.offset = take_offsets(1);
   Tensor y;
+  Buffer buffer;
   std::shared_ptr<HotLinearBackward> node;
   const bool data_grads = wants_grad(x) || wants_grad(w);
   if (data_grads || wants_grad(bias)) node.reset(new HotLinearBackward(), torch::autograd::deleteNode);
@@ -423,7 +436,7 @@ PyObject* linear_impl(PyObject* const* a) {
     pybind11::gil_scoped_release no_gil;
     at::AutoDispatchBelowADInplaceOrView below;
     c10::cuda::CUDAGuard guard(x.device());
-    if (data_grads) compress(l, x.contiguous(), node->s);
+    if (data_grads) buffer = compress(l, x.contiguous());
     // 16-bit tensors: the bias goes into the forward GEMM (one rounding of the output); float32 keeps the reference's
     // separate addition, whose result the parity tests pin bit for bit
     const bool fused = bias.defined() && l.cfg.dtype == HOT_BF16;
@@ -434,7 +447,7 @@ PyObject* linear_impl(PyObject* const* a) {
       else y.add_(bias);
     }
   }
-  if (node) attach(node, y, x, w, bias, a[6]);
+  if (node) attach(node, y, x, w, bias, l, buffer, a[6]);
   return THPVariable_Wrap(y);
 }
 
@@ -465,6 +478,7 @@ PyObject* conv2d_impl(PyObject* const* a) {
   if (preset && l.cfg.q_x.bits <= 4) l.cfg.q_x.storage = HOT_STORE_INT4;
   l.cfg.q_x.offset = take_offsets(1);
   Tensor y;
+  Buffer buffer;
   std::shared_ptr<HotConvBackward> node;
   const bool data_grads = wants_grad(x) || wants_grad(w);
   if (data_grads || wants_grad(bias)) {
@@ -478,14 +492,14 @@ PyObject* conv2d_impl(PyObject* const* a) {
     c10::cuda::CUDAGuard guard(x.device());
     const Tensor xc = x.contiguous(), cols = at::empty({v.B, positions, l.I}, x.options());
     check(hot_im2col(&v, xc.data_ptr(), cols.data_ptr(), current_stream()), "hot_im2col");
-    if (data_grads) compress(l, cols, node->s);
+    if (data_grads) buffer = compress(l, cols);
     const Tensor rows = at::linear(cols, w.view({l.O, l.I}));
     TORCH_CHECK(rows.scalar_type() == x.scalar_type() && rows.is_contiguous(), "HQ_Conv2d: the product came back in another type or layout");
     y = at::empty({v.B, l.O, oh, ow}, x.options());
     check(hot_transpose(v.dtype, v.B, positions, l.O, rows.data_ptr(), bias.defined() ? bias.data_ptr() : nullptr, y.data_ptr(), current_stream()),
           "hot_transpose");
   }
-  if (node) attach(node, y, x, w, bias, a[6]);
+  if (node) attach(node, y, x, w, bias, l, buffer, a[6]);
   return THPVariable_Wrap(y);
 }
 
