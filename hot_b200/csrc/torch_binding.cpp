@@ -7,18 +7,22 @@
 // backward, as the reference does, allocates through torch's caching allocator and makes one C call per direction.
 //
 // linear() and conv2d() answer None for whatever it does not cover (other transform schemes, the logarithmic quantiser, token
-// bases above 64, other dtypes or devices, autocast, arguments that are in error); the caller then takes the Python Function,
+// bases above 64, other dtypes or devices, autocast, tracing, functorch transforms, forward-mode gradients, tensor
+// subclasses and dispatch modes, arguments that are in error); the caller then takes the Python Function,
 // which covers or refuses it.  A configuration that leaves the covered set between forward and backward
 // goes to that Function's backward too.
 #include <torch/extension.h>
 
+#include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/autocast_mode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/Exceptions.h>
 
 #include "hot_b200.h"
@@ -346,22 +350,31 @@ struct HotConvBackward : public Node {
   }
 };
 
+// Whether torch has to see the operations of a call one by one: kernels launched on raw pointers would be missing from a
+// trace or a dispatch mode's record, lose a tangent, or meet a wrapper that has no memory.
+bool seen_by_torch(const Tensor& t) { return at::isTensorSubclassLike(t) || t._fw_grad(0).defined(); }
+bool torch_watches() {
+  return torch::jit::tracer::isTracing() || c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+}
+
 // The part of a layer's configuration that forward fixes; false: not covered (a Python error may be pending).
 // a: x, w, bias or None, order_o, order_l, selection, name
 bool forward_config(PyObject* const* a, hot_linear_cfg_t& c, bool& preset) {
   if (at::autocast::is_autocast_enabled(at::kCUDA)) return false;  // the product would come in autocast's type, not the tensors'
+  if (torch_watches()) return false;
   if (!THPVariable_Check(a[0]) || !THPVariable_Check(a[1]) || !PyList_Check(a[5])) return false;
   const Tensor &x = THPVariable_Unpack(a[0]), &w = THPVariable_Unpack(a[1]);
   const int dt = dtype_code(x.scalar_type());
   const Py_ssize_t rank = PyList_GET_SIZE(a[5]);
   const long order_o = PyLong_AsLong(a[3]), order_l = PyLong_AsLong(a[4]);
   if (PyErr_Occurred()) return false;
+  if (seen_by_torch(x) || seen_by_torch(w)) return false;
   if (!x.is_cuda() || !w.is_cuda() || dt < 0 || x.scalar_type() != w.scalar_type() || x.device() != w.device() || x.numel() == 0 ||
       order_l < 1 || order_l > 64 || order_o < 1 || order_o > 16 || rank < 1 || rank > 64)
     return false;
   if (a[2] != Py_None) {
     const Tensor& bias = THPVariable_Unpack(a[2]);
-    if (!bias.is_cuda() || bias.scalar_type() != x.scalar_type()) return false;
+    if (seen_by_torch(bias) || !bias.is_cuda() || bias.scalar_type() != x.scalar_type()) return false;
   }
   Ref mod(PyObject_CallMethodNoArgs(g_qm, N.args_fn));
   if (!mod || !scheme_covered(mod.p)) return false;
