@@ -374,7 +374,7 @@ bool forward_config(PyObject* const* a, hot_linear_cfg_t& c, bool& preset) {
     return false;
   if (a[2] != Py_None) {
     const Tensor& bias = THPVariable_Unpack(a[2]);
-    if (seen_by_torch(bias) || !bias.is_cuda() || bias.scalar_type() != x.scalar_type()) return false;
+    if (seen_by_torch(bias) || bias.device() != x.device() || bias.scalar_type() != x.scalar_type()) return false;
   }
   Ref mod(PyObject_CallMethodNoArgs(g_qm, N.args_fn));
   if (!mod || !scheme_covered(mod.p)) return false;
@@ -455,7 +455,7 @@ PyObject* linear_impl(PyObject* const* a) {
     const bool fused = bias.defined() && l.cfg.dtype == HOT_BF16;
     y = fused ? at::linear(x, w, bias) : at::linear(x, w);
     if (bias.defined() && !fused) {
-      if (y.scalar_type() == at::kFloat && y.is_contiguous() && bias.is_contiguous() && bias.numel() == l.O && bias.device() == y.device())
+      if (y.scalar_type() == at::kFloat && y.is_contiguous() && bias.is_contiguous() && bias.numel() == l.O)
         check(hot_add_bias((float*)y.data_ptr(), (const float*)bias.data_ptr(), y.numel() / l.O, l.O, current_stream()), "hot_add_bias");
       else y.add_(bias);
     }
@@ -472,6 +472,7 @@ PyObject* conv2d_impl(PyObject* const* a) {
   const Tensor x = THPVariable_Unpack(a[0]), w = THPVariable_Unpack(a[1]);
   const Tensor bias = a[2] == Py_None ? Tensor() : THPVariable_Unpack(a[2]);
   if (x.dim() != 4 || w.dim() != 4 || x.size(1) != w.size(1) || !w.is_contiguous()) return Py_NewRef(Py_None);
+  if (bias.defined() && (bias.dim() != 1 || bias.size(0) != w.size(0) || !bias.is_contiguous())) return Py_NewRef(Py_None);  // (read as it lies)
   hot_conv_t v = {};
   v.dtype = l.cfg.dtype;
   v.B = x.size(0); v.C = x.size(1); v.H = x.size(2); v.W = x.size(3);
