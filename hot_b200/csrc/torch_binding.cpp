@@ -143,15 +143,16 @@ bool scheme_covered(PyObject* mod) {
   return attr_true(mod, N.t_gogi) && attr_true(mod, N.t_wgt) && attr_true(mod, N.t_gogw) && attr_true(mod, N.t_input);
 }
 
+// int(SEED or 0), whatever number SEED is; a Python error may be pending.
 uint64_t seed_of(PyObject* mod) {
   Ref v(PyObject_GetAttr(mod, N.seed));
   if (!v) {
     PyErr_Clear();
     return 0;
   }
-  const uint64_t s = PyLong_Check(v.p) ? PyLong_AsUnsignedLongLongMask(v.p) : 0;
-  if (PyErr_Occurred()) PyErr_Clear();
-  return s;
+  if (PyObject_IsTrue(v.p) != 1) return 0;
+  Ref n(PyNumber_Long(v.p));
+  return n ? PyLong_AsUnsignedLongLongMask(n.p) : 0;
 }
 
 // Takes `count` offsets from the module's Philox call counter; the first of them.
@@ -194,7 +195,9 @@ bool backward_quantisers(PyObject* layer_name, hot_linear_cfg_t& c) {
               !quantiser_attr(mod.p, N.q_gogw, attr_int(mod.p, N.b_gogw), true, false, c.q_gw)))
     return false;
   if (!quantiser_attr(mod.p, N.q_wgt, attr_int(mod.p, N.b_wgt), false, true, c.q_w)) return false;
-  const uint64_t seed = seed_of(mod.p), first = take_offsets(3);
+  const uint64_t seed = seed_of(mod.p);
+  if (PyErr_Occurred()) throw_python();
+  const uint64_t first = take_offsets(3);
   c.q_gx.seed = c.q_gw.seed = c.q_w.seed = seed;
   c.q_gx.offset = first;
   c.q_gw.offset = first + 1;
@@ -388,7 +391,7 @@ bool forward_config(PyObject* const* a, hot_linear_cfg_t& c, bool& preset) {
   if (!v) PyErr_Clear();
   preset = v && v.p != Py_None;
   c.q_x.seed = seed_of(mod.p);
-  return true;
+  return !PyErr_Occurred();
 }
 
 // The activation buffer, made from the rows of x (contiguous).
