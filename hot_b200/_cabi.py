@@ -101,6 +101,7 @@ EXPORTS = {
     "hot_layer_compress_workspace_bytes": (ctypes.c_size_t, [ctypes.POINTER(HotLayer)]),
     "hot_layer_compress": (ctypes.c_int, [ctypes.POINTER(HotLayer), c_vp, c_i64, c_vp, c_vp, c_vp, ctypes.c_size_t, c_vp]),
     "hot_layer_backward_workspace_bytes": (ctypes.c_size_t, [ctypes.POINTER(HotLayer)]),
+    "hot_layer_sums_rows": (ctypes.c_int, [ctypes.POINTER(HotLayer), c_vp]),
     "hot_layer_backward": (ctypes.c_int, [ctypes.POINTER(HotLayer), c_vp, c_vp, c_i64, c_vp, c_vp, c_vp, c_i64, c_vp, c_i64, c_vp, c_vp,
                                           ctypes.c_size_t, c_vp, c_vp]),
     "hot_im2col": (ctypes.c_int, [ctypes.POINTER(HotConv), c_vp, c_vp, c_vp]),

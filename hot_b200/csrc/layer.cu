@@ -260,7 +260,7 @@ int layer_backward(const hot_layer_t& l, const void* go, int64_t ldgo, const voi
     times16 = row && c.q_gx.bits == 4 && c.q_gx.rounding == HOT_ROUND_STOCH_PHILOX && c.q_gx.storage == HOT_STORE_INT8;
     jgo.times16 = times16;
     if (row || col || sum_only) {
-      if (!tile_job_covered(jgo, c.dtype)) HOT_FAIL(HOT_ERR_UNSUPPORTED, "hot_layer_backward: the sum of grad_out's rows needs an even number of channels");
+      if (!tile_job_covered(jgo, c.dtype)) HOT_FAIL(HOT_ERR_UNSUPPORTED, "hot_layer_backward: grad_b is not made for this grad_out (see hot_layer_sums_rows)");
       jobs[count++] = jgo;
     }
     const bool weight = grad_x && tile_job_covered(jw, c.dtype);
@@ -403,6 +403,15 @@ extern "C" size_t hot_layer_backward_workspace_bytes(const hot_layer_t* layer) {
   if (check_layer(layer, "hot_layer_backward_workspace_bytes")) return 0;
   Plan p;
   return make_plan(*layer, p) ? 0 : p.total;
+}
+
+extern "C" int hot_layer_sums_rows(const hot_layer_t* layer, const void* go) {
+  using namespace hot;
+  Plan p;
+  if (check_layer(layer, "hot_layer_sums_rows") || make_plan(*layer, p)) return 0;
+  TileJob jgo, jw;
+  backward_jobs(*layer, p, go, layer->O, nullptr, layer->I, nullptr, false, false, &p, jgo, jw);  // (any non-null sum)
+  return tile_job_covered(jgo, layer->cfg.dtype) ? 1 : 0;
 }
 
 extern "C" int hot_layer_backward(const hot_layer_t* layer, const void* go, const void* w, int64_t ldw, const void* x_q_t,

@@ -371,7 +371,8 @@ int hot_linear_backward(const void* go, int64_t ldgo, const void* w, int64_t ldw
  *              sample and row / channel), grad_w summed over the samples (utils/quant_matmul.py:180,223-225,288-290,322-324)
  * x, go and grad_x have batch * L (batch 0: L) rows; go is contiguous.  The activation buffer is
  * [I, hot_layer_buffer_pitch] bytes with max(batch, 1) scales; a workspace is 256-byte aligned.  grad_b (may be NULL)
- * is the bias gradient, the sum of go over its rows [O].  The size functions
+ * is the bias gradient, the sum of go over its rows [O]; hot_layer_sums_rows says (1 or 0) whether it is made for this go,
+ * which takes an even O and channel pairs that can be loaded at once.  The size functions
  * return 0 for a layer that is not covered (hot_last_error says why).
  */
 typedef struct hot_layer {
@@ -383,6 +384,7 @@ size_t hot_layer_compress_workspace_bytes(const hot_layer_t* layer);
 int hot_layer_compress(const hot_layer_t* layer, const void* x, int64_t ldx, void* x_q_t, float* scale_x, void* workspace,
                        size_t workspace_bytes, hot_stream_t stream);
 size_t hot_layer_backward_workspace_bytes(const hot_layer_t* layer);
+int hot_layer_sums_rows(const hot_layer_t* layer, const void* go);
 int hot_layer_backward(const hot_layer_t* layer, const void* go, const void* w, int64_t ldw, const void* x_q_t,
                        const float* scale_x, void* grad_x, int64_t ldgx, void* grad_w, int64_t ldgw, void* grad_b,
                        void* workspace, size_t workspace_bytes, uint32_t* status_word, hot_stream_t stream);
