@@ -13,6 +13,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kSmemLimit = 96 * 1024;  // two CTAs per SM
+constexpr int kMaxGridY = 65535;
 
 struct ConvGeo {
   int C, H, W, OH, OW, kh, kw, sh, sw, ph, pw, dh, dw;
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(kThreads) im2col_kernel(const R* __restrict__ 
   }
 }
 
-// Rows too long for shared memory: one element per thread, read where it lies.
+// Rows too long for shared memory, or too many of them for a launch: one element per thread, read where it lies.
 template <typename R>
 __global__ void __launch_bounds__(kThreads) im2col_direct_kernel(const R* __restrict__ x, R* __restrict__ cols, ConvGeo g) {
   const int64_t ckk = (int64_t)g.C * g.kk, total = (int64_t)g.OH * g.OW * ckk;
@@ -195,41 +196,46 @@ __global__ void __launch_bounds__(kThreads) col2im_kernel(const R* __restrict__ 
 
 // out[b][c][r] = in[b][r][c] (+ bias[c], rounded once more, as a separate addition would): 64 x 64 tiles, neighbouring
 // lanes on neighbouring elements on both sides.  VI / VO: 16-bit elements per load / store (pairs where the rows of that
-// side begin at whole words: 6.4 MB transposed in 7.3 us one by one).
+// side begin at whole words: 6.4 MB transposed in 7.3 us one by one).  A CTA takes every gridDim.y-th tile of its columns.
 template <typename R, int VI, int VO>
 __global__ void __launch_bounds__(kThreads) transpose_kernel(const R* __restrict__ in, const R* __restrict__ bias, R* __restrict__ out,
                                                              int rows, int cols) {
   __shared__ __align__(16) R tile[64][sizeof(R) == 2 ? 66 : 65];
-  const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
+  const int c0 = blockIdx.x * 64;
   in += (int64_t)blockIdx.z * rows * cols;
   out += (int64_t)blockIdx.z * rows * cols;
   constexpr int kLanesI = 64 / VI, kLanesO = 64 / VO;
-  {
-    const int tx = threadIdx.x % kLanesI * VI, ty = threadIdx.x / kLanesI;
+  for (int r0 = blockIdx.y * 64;;) {
+    {
+      const int tx = threadIdx.x % kLanesI * VI, ty = threadIdx.x / kLanesI;
 #pragma unroll
-    for (int i = 0; i < 64 * kLanesI / kThreads; ++i) {
-      const int rr = ty + i * (kThreads / kLanesI), r = r0 + rr, c = c0 + tx;
-      if (r < rows && c < cols) {
-        if constexpr (VI == 2) *reinterpret_cast<uint32_t*>(&tile[rr][tx]) = __ldg(reinterpret_cast<const uint32_t*>(in + (int64_t)r * cols + c));
-        else tile[rr][tx] = __ldg(in + (int64_t)r * cols + c);
+      for (int i = 0; i < 64 * kLanesI / kThreads; ++i) {
+        const int rr = ty + i * (kThreads / kLanesI), r = r0 + rr, c = c0 + tx;
+        if (r < rows && c < cols) {
+          if constexpr (VI == 2) *reinterpret_cast<uint32_t*>(&tile[rr][tx]) = __ldg(reinterpret_cast<const uint32_t*>(in + (int64_t)r * cols + c));
+          else tile[rr][tx] = __ldg(in + (int64_t)r * cols + c);
+        }
       }
     }
-  }
-  __syncthreads();
-  const int tx = threadIdx.x % kLanesO * VO, ty = threadIdx.x / kLanesO;
+    __syncthreads();
+    const int tx = threadIdx.x % kLanesO * VO, ty = threadIdx.x / kLanesO;
 #pragma unroll
-  for (int i = 0; i < 64 * kLanesO / kThreads; ++i) {
-    const int cc = ty + i * (kThreads / kLanesO), c = c0 + cc, r = r0 + tx;
-    if (c < cols && r < rows) {
-      R v[VO];
+    for (int i = 0; i < 64 * kLanesO / kThreads; ++i) {
+      const int cc = ty + i * (kThreads / kLanesO), c = c0 + cc, r = r0 + tx;
+      if (c < cols && r < rows) {
+        R v[VO];
 #pragma unroll
-      for (int k = 0; k < VO; ++k) {
-        v[k] = tile[tx + k][cc];
-        if (bias) v[k] = narrow<R>(__fadd_rn(widen(v[k]), widen(bias[c])));
+        for (int k = 0; k < VO; ++k) {
+          v[k] = tile[tx + k][cc];
+          if (bias) v[k] = narrow<R>(__fadd_rn(widen(v[k]), widen(bias[c])));
+        }
+        if constexpr (VO == 2) *reinterpret_cast<uint32_t*>(out + (int64_t)c * rows + r) = (uint32_t)v[0] | ((uint32_t)v[1] << 16);
+        else out[(int64_t)c * rows + r] = v[0];
       }
-      if constexpr (VO == 2) *reinterpret_cast<uint32_t*>(out + (int64_t)c * rows + r) = (uint32_t)v[0] | ((uint32_t)v[1] << 16);
-      else out[(int64_t)c * rows + r] = v[0];
     }
+    r0 += (int)gridDim.y * 64;
+    if (r0 >= rows) break;
+    __syncthreads();
   }
 }
 
@@ -290,7 +296,7 @@ int im2col_typed(const R* x, R* cols, ConvGeo g, int64_t B, cudaStream_t st) {
     else if (g.rows > 1) g.rows = (g.rows + 1) / 2;
     else g.cc = (g.cc + 1) / 2;
   }
-  if (smem() > (size_t)kSmemLimit || (int64_t)g.cc * g.span_h * g.span_w >= 65536) {
+  if (smem() > (size_t)kSmemLimit || (int64_t)g.cc * g.span_h * g.span_w >= 65536 || (g.OH + g.rows - 1) / g.rows > kMaxGridY) {
     im2col_direct_kernel<R><<<dim3(2048, (unsigned)B), kThreads, 0, st>>>(x, cols, g);
     HOT_CUDA(cudaGetLastError());
     return HOT_OK;
@@ -305,7 +311,6 @@ int im2col_typed(const R* x, R* cols, ConvGeo g, int64_t B, cudaStream_t st) {
 template <typename R, int V>
 int launch_col2im(const R* cols, R* x, const ConvGeo& g, int64_t B, size_t bytes, bool staged, cudaStream_t st) {
   const dim3 grid((g.C + g.cc - 1) / g.cc, (g.H + g.rows - 1) / g.rows, (unsigned)B);
-  if (grid.y > 65535) HOT_FAIL(HOT_ERR_UNSUPPORTED, "hot_col2im: image too tall");
   auto launch = [&](auto kernel, PerDeviceOnce& once) -> int {
     if (int rc = allow_smem(kernel, once)) return rc;
     kernel<<<grid, kThreads, staged ? bytes : 0, st>>>(cols, x, g);
@@ -322,7 +327,8 @@ int launch_col2im(const R* cols, R* x, const ConvGeo& g, int64_t B, size_t bytes
 template <typename R>
 int col2im_typed(const R* cols, R* x, ConvGeo g, int64_t B, cudaStream_t st) {
   // Channels per CTA: whole 16-byte vectors, at least 128 contiguous bytes of taps per position.  Rows per CTA: of what
-  // fits, the height that loses least to staging rows twice and to a last round of input elements that is not full.
+  // fits, the height that loses least to staging rows twice and to a last round of input elements that is not full (at
+  // least what keeps the launch within its limits).
   constexpr int kV = 16 / sizeof(R);
   g.cc = (int)((128 / sizeof(R) + g.kk - 1) / g.kk);
   g.cc = (g.cc + kV - 1) / kV * kV;
@@ -335,10 +341,11 @@ int col2im_typed(const R* cols, R* x, ConvGeo g, int64_t B, cudaStream_t st) {
     return ((size_t)g.span_h * g.OW + 1) * words * 4;
   };
   const size_t budget = 72 * 1024;  // three CTAs per SM
-  while (smem(1) > budget && g.cc > 1) g.cc = g.cc > kV ? (g.cc / 2 + kV - 1) / kV * kV : (g.cc + 1) / 2;
+  const int least = (g.H + kMaxGridY - 1) / kMaxGridY;
+  while (smem(least) > budget && g.cc > 1) g.cc = g.cc > kV ? (g.cc / 2 + kV - 1) / kV * kV : (g.cc + 1) / 2;
   double best = -1.0;
-  g.rows = 1;
-  for (int rows = 1; rows <= g.H && (rows == 1 || smem(rows) <= budget); ++rows) {
+  g.rows = least;
+  for (int rows = least; rows <= g.H && (rows == least || smem(rows) <= budget); ++rows) {
     const int tiles = (g.H + rows - 1) / rows, items = rows * g.W;
     const double useful = (double)g.H / ((double)tiles * (rows + (g.kh - 1) * g.dh)) * items / ((items + kThreads - 1) / kThreads * kThreads);
     if (useful > best) {
@@ -350,7 +357,7 @@ int col2im_typed(const R* cols, R* x, ConvGeo g, int64_t B, cudaStream_t st) {
   const bool staged = bytes <= (size_t)kSmemLimit;
   if (!staged) {
     g.cc = g.C < 8 ? g.C : 8;
-    g.rows = 1;
+    g.rows = least;
   }
   g.by_w = fast_div(g.W);
   const bool vec = (int64_t)g.C * g.kk % kV == 0 && (g.cc == g.C || (int64_t)g.cc * g.kk % kV == 0) && ((uintptr_t)cols) % 16 == 0;
@@ -452,9 +459,10 @@ extern "C" int hot_transpose(int dtype, int64_t batch, int64_t rows, int64_t col
                              hot_stream_t stream) {
   using namespace hot;
   if (!in || !out) HOT_FAIL(HOT_ERR_ARG, "hot_transpose: null pointer");
-  if (batch <= 0 || batch > 65535 || rows <= 0 || cols <= 0 || cols > (1 << 30) || rows > 65535ll * 64)
+  if (batch <= 0 || batch > 65535 || rows <= 0 || cols <= 0 || cols > (1 << 30) || rows > (1 << 30))
     HOT_FAIL(HOT_ERR_ARG, "hot_transpose: bad shape");
-  const dim3 grid((unsigned)((cols + 63) / 64), (unsigned)((rows + 63) / 64), (unsigned)batch);
+  const int64_t row_tiles = (rows + 63) / 64;
+  const dim3 grid((unsigned)((cols + 63) / 64), (unsigned)(row_tiles < kMaxGridY ? row_tiles : kMaxGridY), (unsigned)batch);
   cudaStream_t st = (cudaStream_t)stream;
   if (dtype == HOT_F32) {
     transpose_kernel<uint32_t, 1, 1><<<grid, kThreads, 0, st>>>((const uint32_t*)in, (const uint32_t*)bias, (uint32_t*)out, (int)rows, (int)cols);

@@ -488,6 +488,7 @@ PyObject* conv2d_impl(PyObject* const* a) {
   const int64_t oh = (v.H + 2 * v.ph - v.dh * (v.kh - 1) - 1) / v.sh + 1, ow = (v.W + 2 * v.pw - v.dw * (v.kw - 1) - 1) / v.sw + 1;
   if (v.H + 2 * v.ph < v.dh * (v.kh - 1) + 1 || v.W + 2 * v.pw < v.dw * (v.kw - 1) + 1 || v.B > 65535) return Py_NewRef(Py_None);
   const int64_t positions = oh * ow;
+  if (positions > (1 << 30) || v.C * v.kh * v.kw > (1 << 30)) return Py_NewRef(Py_None);
   l.batch = preset ? 0 : v.B;
   l.L = preset ? v.B * positions : positions;
   l.I = v.C * v.kh * v.kw;
