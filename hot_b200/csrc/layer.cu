@@ -471,7 +471,11 @@ extern "C" int hot_hlq_backward(const void* go, const void* w, const void* x, in
   const CompressArgs compress = {x, I, base, scale_x, base + p.off_cws, p.cws};
   const int rc = layer_backward(p.layer, go, O, w, I, base, scale_x, grad_x, I, grad_w, I, nullptr, base + p.off_bws, p.bws, kit->status, kit->ev[1],
                                 stream, &compress);
-  if (rc) return rc;
+  if (rc) {  // refused after launches perhaps: they may still write the status word, which the thread's next call reads
+    cudaStreamSynchronize(st);
+    *kit->status = 0;
+    return rc;
+  }
   HOT_CUDA(cudaEventRecord(kit->ev[2], st));
   HOT_CUDA(cudaStreamSynchronize(st));
   const uint32_t status = *kit->status;
