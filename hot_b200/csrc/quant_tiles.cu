@@ -395,10 +395,18 @@ __device__ __forceinline__ uint4 philox_codes16(const uint32_t (&k)[16], const Q
   }
 }
 
+// max(|a|, |b|, |c|), NaN if any of them is
+__device__ __forceinline__ float absmax3_nan(float a, float b, float c) {
+  float m;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+  return m;
+}
+
 // 16 consecutive codes of two neighbouring channels: y[i] = (value i of channel c, value i of channel c + 1); e_a / e_b:
 // Philox index of the first code of either.
-// Nearest: the quotient (exact, as everywhere) plus 1.5 * 2^23 rounds half to even and leaves the code in the low byte; the
-// largest quotient is qmax within an ulp, so nothing is left to clamp.
+// Nearest: the quotient (exact, as everywhere) plus 1.5 * 2^23 rounds half to even and leaves the code in the low byte.  The
+// largest quotient is qmax within an ulp unless the tensor holds NaN or the scale is none (infinite, or the clip of a tensor of
+// constant magnitude, which is negative): where a quotient of the 32 is beyond, all are done again by the rule with the clamp.
 template <int KIND>
 __device__ __forceinline__ void quantise_pair16(const float2 (&y)[16], const ScalePair& sa, const ScalePair& sb, const QuantDev& q, uint64_t e_a,
                                                 uint64_t e_b, uint4& out_a, uint4& out_b) {
@@ -415,12 +423,21 @@ __device__ __forceinline__ void quantise_pair16(const float2 (&y)[16], const Sca
     out_b = philox_codes16<KIND>(kb, q, e_b);
   } else {
     const float2 r2 = make_float2(sa.dv.r, sb.dv.r), nd2 = make_float2(-sa.dv.d, -sb.dv.d), magic = make_float2(kKMagic, kKMagic);
+    float largest = 0.0f;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const float2 q0 = __fmul2_rn(y[i], r2);
-      const float2 t = add2(__ffma2_rn(__ffma2_rn(q0, nd2, y[i]), r2, q0), magic);
+      const float2 q0 = __fmul2_rn(y[i], r2), f = __ffma2_rn(__ffma2_rn(q0, nd2, y[i]), r2, q0);
+      largest = absmax3_nan(largest, f.x, f.y);
+      const float2 t = add2(f, magic);
       ka[i] = __float_as_uint(t.x);
       kb[i] = __float_as_uint(t.y);
+    }
+    if (!(largest < q.qmax + 0.5f)) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        ka[i] = (uint32_t)quantise_one<HOT_ROUND_NEAREST>(y[i].x, sa, 0.0f, (int)q.qmax);
+        kb[i] = (uint32_t)quantise_one<HOT_ROUND_NEAREST>(y[i].y, sb, 0.0f, (int)q.qmax);
+      }
     }
     out_a = make_uint4(gather_low_bytes(ka[0], ka[1], ka[2], ka[3]), gather_low_bytes(ka[4], ka[5], ka[6], ka[7]),
                        gather_low_bytes(ka[8], ka[9], ka[10], ka[11]), gather_low_bytes(ka[12], ka[13], ka[14], ka[15]));
