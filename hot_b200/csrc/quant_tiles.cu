@@ -348,11 +348,10 @@ __device__ __forceinline__ uint4 philox_bytes_unaligned(const QuantDev& q, uint6
 // Philox with 8-bit or 4-bit codes whose runs begin at whole runs of the random stream, to nearest, or anything.
 enum CodeKind { kCodeAny = 0, kCode8 = 1, kCode4 = 2, kCodeNearest = 3 };
 
-// byte-wide offset codes -> codes, sign-extended where they are narrower than the byte (off = 2^(bits-1))
-__device__ __forceinline__ uint32_t finish4(uint32_t w, uint32_t off, uint32_t shift, uint32_t fill) {
-  const uint32_t sign = off * 0x01010101u;
-  w ^= sign;
-  return w | (((w & sign) >> shift) * fill);
+// offset codes of 4 bits, one per byte -> sign-extended codes
+__device__ __forceinline__ uint32_t finish_nibbles(uint32_t w) {
+  w ^= 0x08080808u;
+  return w | (((w & 0x08080808u) >> 3) * 0xF0u);
 }
 
 template <int KIND>
@@ -367,30 +366,50 @@ __device__ __forceinline__ uint4 philox_codes16(const uint32_t (&k)[16], const Q
     philox_run_words4(q, e0, r0, r1);
     philox_run16_words(k, k + 8, true, r0, r1, 0u, 0u, w[0], w[1], w[2], w[3]);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = finish4((w[i] >> 4) & 0x0F0F0F0Fu, 8u, 3, 0xF0u);
+    for (int i = 0; i < 4; ++i) w[i] = finish_nibbles((w[i] >> 4) & 0x0F0F0F0Fu);
     return make_uint4(w[0], w[1], w[2], w[3]);
   } else {
+    // Sums in packed lanes on runs of 8, one by one elsewhere, as col_ht_quant does: the two differ in what the overflowing sum
+    // of a NaN leaves.
     uint32_t w[4];
-    const uint32_t off = (uint32_t)(q.qmax + 1.0f), shift = 31 - __clz(off), fill = 0x100u - 2u * off;
+    const uint32_t off = (uint32_t)(q.qmax + 1.0f);
+    const bool runs8 = (e0 & 7u) == 0;
     if (rand_bits(q.qmax) == 8) {
       const uint4 r = (e0 & 15u) == 0 ? philox_block(q, e0 >> 4) : philox_bytes_unaligned(q, e0);
-      w[0] = offset_codes4_rb8(k[0], k[1], k[2], k[3], r.x);
-      w[1] = offset_codes4_rb8(k[4], k[5], k[6], k[7], r.y);
-      w[2] = offset_codes4_rb8(k[8], k[9], k[10], k[11], r.z);
-      w[3] = offset_codes4_rb8(k[12], k[13], k[14], k[15], r.w);
+      const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
+      if (runs8) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = offset_codes4_rb8(k[4 * i], k[4 * i + 1], k[4 * i + 2], k[4 * i + 3], rw[i]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          auto one = [&](int j) { return ((k[4 * i + j] & 0xFFFFu) + ((rw[i] >> (8 * j)) & 0xFFu)) >> 8; };
+          w[i] = gather_low_bytes(one(0), one(1), one(2), one(3));
+        }
+      }
     } else {
       const uint4 a = philox_block(q, e0 >> 5), b = philox_block(q, (e0 + 15) >> 5);
-      uint32_t c[16];
+      if (runs8) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const uint64_t e = e0 + (uint64_t)i;
-        c[i] = ((k[i] & 0xFFFFu) + philox_r4((e >> 5) == (e0 >> 5) ? a : b, e)) >> 4;
+        for (int i = 0; i < 4; ++i) {
+          const uint64_t e = e0 + (uint64_t)(4 * i);
+          const uint4 blk = (e >> 5) == (e0 >> 5) ? a : b;
+          const uint32_t word = (e & 16u) ? ((i & 1) ? blk.w : blk.z) : ((i & 1) ? blk.y : blk.x);
+          w[i] = (offset_sums4_rb4(k[4 * i], k[4 * i + 1], k[4 * i + 2], k[4 * i + 3], (word >> ((e & 8u) ? 4 : 0)) & 0x0F0F0F0Fu) >> 4) & 0x0F0F0F0Fu;
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          auto one = [&](int j) {
+            const uint64_t e = e0 + (uint64_t)(4 * i + j);
+            return ((k[4 * i + j] & 0xFFFFu) + philox_r4((e >> 5) == (e0 >> 5) ? a : b, e)) >> 4;
+          };
+          w[i] = gather_low_bytes(one(0), one(1), one(2), one(3));
+        }
       }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) w[i] = gather_low_bytes(c[4 * i], c[4 * i + 1], c[4 * i + 2], c[4 * i + 3]);
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = finish4(w[i], off, shift, fill);
+    for (int i = 0; i < 4; ++i) w[i] = __vsub4(w[i], off * 0x01010101u);
     return make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
@@ -402,13 +421,15 @@ __device__ __forceinline__ float absmax3_nan(float a, float b, float c) {
   return m;
 }
 
+__device__ __forceinline__ float code_range(float v, float qmax) { return v == v ? fminf(fmaxf(v, -qmax), qmax) : 0.0f; }
+
 // 16 consecutive codes of two neighbouring channels: y[i] = (value i of channel c, value i of channel c + 1); e_a / e_b:
 // Philox index of the first code of either.
 // Nearest: the quotient (exact, as everywhere) plus 1.5 * 2^23 rounds half to even and leaves the code in the low byte.  The
 // largest quotient is qmax within an ulp unless the tensor holds NaN or the scale is none (infinite, or the clip of a tensor of
-// constant magnitude, which is negative): where a quotient of the 32 is beyond, all are done again by the rule with the clamp.
+// constant magnitude, which is negative): where one of the 32 is beyond, they are clamped, and a NaN gives code 0.
 template <int KIND>
-__device__ __forceinline__ void quantise_pair16(const float2 (&y)[16], const ScalePair& sa, const ScalePair& sb, const QuantDev& q, uint64_t e_a,
+__device__ __forceinline__ void quantise_pair16(float2 (&y)[16], const ScalePair& sa, const ScalePair& sb, const QuantDev& q, uint64_t e_a,
                                                 uint64_t e_b, uint4& out_a, uint4& out_b) {
   uint32_t ka[16], kb[16];
   if constexpr (KIND != kCodeNearest) {
@@ -426,18 +447,19 @@ __device__ __forceinline__ void quantise_pair16(const float2 (&y)[16], const Sca
     float largest = 0.0f;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const float2 q0 = __fmul2_rn(y[i], r2), f = __ffma2_rn(__ffma2_rn(q0, nd2, y[i]), r2, q0);
-      largest = absmax3_nan(largest, f.x, f.y);
-      const float2 t = add2(f, magic);
-      ka[i] = __float_as_uint(t.x);
-      kb[i] = __float_as_uint(t.y);
+      const float2 q0 = __fmul2_rn(y[i], r2);
+      y[i] = __ffma2_rn(__ffma2_rn(q0, nd2, y[i]), r2, q0);
+      largest = absmax3_nan(largest, y[i].x, y[i].y);
     }
     if (!(largest < q.qmax + 0.5f)) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        ka[i] = (uint32_t)quantise_one<HOT_ROUND_NEAREST>(y[i].x, sa, 0.0f, (int)q.qmax);
-        kb[i] = (uint32_t)quantise_one<HOT_ROUND_NEAREST>(y[i].y, sb, 0.0f, (int)q.qmax);
-      }
+      for (int i = 0; i < 16; ++i) y[i] = make_float2(code_range(y[i].x, q.qmax), code_range(y[i].y, q.qmax));
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float2 t = add2(y[i], magic);
+      ka[i] = __float_as_uint(t.x);
+      kb[i] = __float_as_uint(t.y);
     }
     out_a = make_uint4(gather_low_bytes(ka[0], ka[1], ka[2], ka[3]), gather_low_bytes(ka[4], ka[5], ka[6], ka[7]),
                        gather_low_bytes(ka[8], ka[9], ka[10], ka[11]), gather_low_bytes(ka[12], ka[13], ka[14], ka[15]));
