@@ -222,7 +222,7 @@ int layer_backward(const hot_layer_t& l, const void* go, int64_t ldgo, const voi
   const bool gx_row = c.q_gx.scale_mode == HOT_SCALE_ROW;
   hot_quant_t q_w8 = c.q_w;
   q_w8.storage = HOT_STORE_INT8;
-  bool counters_cleared = false, times16 = false;
+  bool counters_cleared = false;
 
   auto compress_alone = [&]() {
     return compress ? hot_layer_compress(&l, compress->x, compress->ldx, compress->x_q_t, compress->scale_x, compress->workspace,
@@ -257,8 +257,7 @@ int layer_backward(const hot_layer_t& l, const void* go, int64_t ldgo, const voi
     if (col && !covered(false, true)) col = false;
     backward_jobs(l, p, go, ldgo, w, ldw, base, row, col, grad_b, jgo, jw);
     const bool sum_only = grad_b && !row && !col;
-    times16 = row && c.q_gx.bits == 4 && c.q_gx.rounding == HOT_ROUND_STOCH_PHILOX && c.q_gx.storage == HOT_STORE_INT8;
-    jgo.times16 = times16;
+    jgo.times16 = row && c.q_gx.bits == 4 && c.q_gx.rounding == HOT_ROUND_STOCH_PHILOX && c.q_gx.storage == HOT_STORE_INT8;
     if (row || col || sum_only) {
       if (!tile_job_covered(jgo, c.dtype)) HOT_FAIL(HOT_ERR_UNSUPPORTED, "hot_layer_backward: grad_b is not made for this grad_out (see hot_layer_sums_rows)");
       jobs[count++] = jgo;
@@ -288,7 +287,7 @@ int layer_backward(const hot_layer_t& l, const void* go, int64_t ldgo, const voi
   }
   if (quantised) HOT_CUDA(cudaEventRecord(quantised, st));
 
-  const float post_x = (times16 ? 0.0625f : 1.0f) / (float)c.order_o, post_w = 1.0f / (float)c.order_l;
+  const float post_x = 1.0f / (float)c.order_o, post_w = 1.0f / (float)c.order_l;
   const int rows_per_scale = gx_row ? 1 : (l.batch ? (int)l.L : 0);
   if (l.batch) {
     if (grad_x)

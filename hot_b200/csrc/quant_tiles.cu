@@ -582,7 +582,9 @@ __device__ __forceinline__ void quant_tile(const DevJob& j, int at, uint8_t* sme
 
   if (!WEIGHT && j.row_on) {
     const ScalePair sp = scale_from_absmax(max_of_partials(j.part_row + (int64_t)b * parts, parts), j.qr.qmax);
-    if (tile == 0 && cb == 0 && threadIdx.x == 0) j.s_row[b] = sp.s;
+    // (16 * code goes with a sixteenth of the scale, exact wherever a code is not 0: their product is the unstored one's, so it
+    // overflows where that does)
+    if (tile == 0 && cb == 0 && threadIdx.x == 0) j.s_row[b] = j.row_store == kRowTimes16 ? 0.0625f * sp.s : sp.s;
     if (j.row_store != kRowTimes16) row_side_any<T>(j, x, b, t0, c0, sp);
     else if (j.n_row == 16 && (j.C & 31) == 0) row_side_times16<T, 16, true>(j, x, b, t0, c0, sp);
     else row_side_times16<T, 0, false>(j, x, b, t0, c0, sp);

@@ -14,7 +14,7 @@ struct TileJob {
   bool row = false;
   int order_row = 1;
   hot_quant_t q_row = {};
-  bool times16 = false;     // 4-bit Philox codes one per byte, stored as 16 * code (the GEMM's post factor takes it back)
+  bool times16 = false;     // 4-bit Philox codes one per byte, stored as 16 * code with the scale / 16
   void* codes_row = nullptr;
   int64_t ld_row = 0;
   float* scale_row = nullptr;
