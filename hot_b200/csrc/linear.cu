@@ -91,6 +91,7 @@ extern "C" int hot_linear_backward(const void* go, int64_t ldgo, const void* w, 
                                    size_t workspace_bytes, uint32_t* status_word, hot_stream_t stream) {
   using namespace hot;
   if (!cfg) HOT_FAIL(HOT_ERR_ARG, "hot_linear_backward: null pointer");
+  if (cfg->order_o > 16) HOT_FAIL(HOT_ERR_ARG, "hot_linear_backward: order_o %d outside [1, 16]", cfg->order_o);  // (the extension call takes up to 64)
   const hot_layer_t layer = {0, L, O, I, *cfg};
   return layer_backward(layer, go, ldgo, w, ldw, x_q_t, scale_x, grad_x, ldgx, grad_w, ldgw, nullptr, workspace, workspace_bytes, status_word,
                         nullptr, stream);

@@ -101,3 +101,18 @@ def test_host_modules_without_a_device():
     from hot_b200.quant_matmul import FLinearQ
     import inspect
     assert list(inspect.signature(FLinearQ.forward).parameters)[:7] == ["ctx", "x", "w", "h_out", "h_bs", "name", "bias"]
+
+
+def test_linear_backward_refuses_orders_above_16(cabi):
+    """Along the output features a layer's transform is of order 16 at most (the extension call alone takes up to 64)."""
+    lib, cfg = cabi.lib(), cabi.HotLinearCfg()
+    cfg.order_o, cfg.order_l, cfg.rank_l = 32, 16, 8
+    for i in range(8):
+        cfg.sel_l[i] = 2 * i
+    for q in (cfg.q_gx, cfg.q_w, cfg.q_gw, cfg.q_x):
+        q.bits = 4
+    L = O = I = 64
+    buf = (ctypes.c_uint8 * (int(lib.hot_linear_workspace_bytes(L, O, I, ctypes.byref(cfg))) + 256))()
+    p = (ctypes.addressof(buf) + 255) // 256 * 256
+    rc = lib.hot_linear_backward(p, O, p, I, p, p, L, O, I, ctypes.byref(cfg), p, I, p, I, p, len(buf) - 256, None, None)
+    assert rc == cabi.HOT_ERR_ARG and b"order_o 32" in lib.hot_last_error()
