@@ -14,6 +14,7 @@ from . import _cabi as C
 from ._native import native
 
 _DTYPES = {torch.float32: C.HOT_F32, torch.bfloat16: C.HOT_BF16}
+_SCALE = {"tensor": C.SCALE_TENSOR, "row": C.SCALE_ROW, "sawb": C.SCALE_SAWB}
 _ROUNDING = {"nearest": C.ROUND_NEAREST, "philox": C.ROUND_STOCH_PHILOX, "noise": C.ROUND_STOCH_NOISE}
 
 
@@ -33,7 +34,7 @@ class Quant:
         q.bits = self.bits
         q.storage = C.STORE_INT4 if self.storage == "int4" else C.STORE_INT8
         q.rounding = _ROUNDING[self.rounding]
-        q.scale_mode = {"tensor": C.SCALE_TENSOR, "row": C.SCALE_ROW, "sawb": C.SCALE_SAWB}[self.scale]
+        q.scale_mode = _SCALE[self.scale]
         q.seed, q.offset = self.seed & (2 ** 64 - 1), self.offset & (2 ** 64 - 1)
         if self.rounding == "noise":
             if self.noise is None or self.noise.dtype != torch.float32 or not self.noise.is_contiguous():
@@ -98,7 +99,8 @@ def row_ht_quant(x: torch.Tensor, order: int, q: Quant):
     noise = 0
     if q.rounding == "noise":
         noise = q.to_c().noise or 0
-    return native().row_ht_quant(x, order, q.bits, q.storage == "int4", _ROUNDING[q.rounding], q.scale == "row", q.seed, q.offset, noise)
+    return native().row_ht_quant(x, order, q.bits, q.storage == "int4", _ROUNDING[q.rounding], _SCALE[q.scale] == C.SCALE_ROW, q.seed,
+                                 q.offset, noise)
 
 
 def col_ht_quant(x: torch.Tensor, order: int, sel: Sequence[int], q: Quant, logical_layout: str = "natural"):

@@ -621,3 +621,10 @@ def test_row_ht_quant_pairs_of_runs(ops, rows, cols, order, lead, dtype, storage
     ref_c, ref_s = (oc.quant_rows if scale == "row" else oc.quant_tensor)(oc.fwht_last(_as_f32(x, dtype), order), bits, oc.philox_bytes(3, 5, x.shape))
     assert np.array_equal(np.atleast_1d(ref_s).astype(np.float32).view(np.uint32), scales.cpu().numpy().view(np.uint32))
     assert np.array_equal(_codes_from(codes, storage, cols), ref_c)
+
+
+def test_row_ht_quant_refuses_unknown_names(ops):
+    x = torch.zeros((4, 64), device="cuda")
+    for q in (ops.Quant(4, "int4", "nearest", "rows"), ops.Quant(4, "int4", "neareast", "row")):
+        with pytest.raises(KeyError):
+            ops.row_ht_quant(x, 16, q)
