@@ -10,6 +10,7 @@ other combination of flags raises; nothing falls back to float emulation.
 from __future__ import annotations
 
 import sys
+import weakref
 from types import SimpleNamespace
 from typing import Optional
 
@@ -252,15 +253,15 @@ _selection_cache: dict = {}
 
 
 def _selection(h_bs: Tensor):
-    """(n, sel) of the low-rank matrix a layer carries; cached on the matrix's identity."""
-    key = (h_bs.data_ptr(), tuple(h_bs.shape), h_bs._version)
-    hit = _selection_cache.get(key)
-    if hit is None:
-        hit = selection_from_matrix(h_bs)
+    """(n, sel) of the low-rank matrix a layer carries; kept while that very tensor lives and is not written to (another
+    matrix may come to lie at its address)."""
+    hit = _selection_cache.get(id(h_bs))
+    if hit is None or hit[0]() is not h_bs or hit[1] != (h_bs.data_ptr(), h_bs._version):
+        hit = (weakref.ref(h_bs), (h_bs.data_ptr(), h_bs._version), selection_from_matrix(h_bs))
         if len(_selection_cache) > 256:
             _selection_cache.clear()
-        _selection_cache[key] = hit
-    return hit
+        _selection_cache[id(h_bs)] = hit
+    return hit[2]
 
 
 class FLinearQ(Function):

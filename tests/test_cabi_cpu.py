@@ -116,3 +116,16 @@ def test_linear_backward_refuses_orders_above_16(cabi):
     p = (ctypes.addressof(buf) + 255) // 256 * 256
     rc = lib.hot_linear_backward(p, O, p, I, p, p, L, O, I, ctypes.byref(cfg), p, I, p, I, p, len(buf) - 256, None, None)
     assert rc == cabi.HOT_ERR_ARG and b"order_o 32" in lib.hot_last_error()
+
+
+def test_kept_selection_of_a_matrix_that_comes_to_lie_where_another_did():
+    import torch
+    from hot_b200.hadamard_matmul import hadamard
+    from hot_b200.quant_matmul import _selection
+    rng = np.random.default_rng(0)
+    for _ in range(64):
+        rows = rng.permutation(16)
+        m = torch.tensor(hadamard(16)[rows].copy())
+        assert list(_selection(m)[1]) == rows.tolist() and list(_selection(m)[1]) == rows.tolist()
+        m.copy_(torch.tensor(hadamard(16)[rows[::-1].copy()]))
+        assert list(_selection(m)[1]) == rows[::-1].tolist()
