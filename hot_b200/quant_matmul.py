@@ -257,11 +257,16 @@ def _selection(h_bs: Tensor):
     matrix may come to lie at its address)."""
     hit = _selection_cache.get(id(h_bs))
     if hit is None or hit[0]() is not h_bs or hit[1] != (h_bs.data_ptr(), h_bs._version):
-        hit = (weakref.ref(h_bs), (h_bs.data_ptr(), h_bs._version), selection_from_matrix(h_bs))
-        if len(_selection_cache) > 256:
-            _selection_cache.clear()
-        _selection_cache[id(h_bs)] = hit
+        return _keep_selection(h_bs, selection_from_matrix(h_bs))
     return hit[2]
+
+
+def _keep_selection(h_bs: Tensor, selection):
+    """Enters what a layer knows of the matrix it just made (reading it back from the device would wait for the device)."""
+    if len(_selection_cache) > 256:
+        _selection_cache.clear()
+    _selection_cache[id(h_bs)] = (weakref.ref(h_bs), (h_bs.data_ptr(), h_bs._version), selection)
+    return selection
 
 
 class FLinearQ(Function):
@@ -512,6 +517,7 @@ class HQ_Linear(nn.Linear):
         if key != self._bs_tokens or self.hadamard_bs.device != self.weight.device:
             n, sel = _token_basis(a, tokens, getattr(a, "lowRankPreset", None))
             self.hadamard_bs = self._basis(n, sel, self.weight.device)
+            _keep_selection(self.hadamard_bs, (n, sel))
             self.hadamard_out = _out_matrix(a, self.out_features, tokens, getattr(a, "lowRankPreset", None),
                                             self.weight.dtype, self.weight.device)
             self._bs_tokens = key
@@ -550,6 +556,7 @@ class HQ_Conv2d(nn.Conv2d):
             from .hadamard_matmul import hadamard
             n, sel = _token_basis(a, tokens, preset)
             self.hadamard_bs = torch.tensor(hadamard(n)[sel], dtype=self.weight.dtype, device=self.weight.device)
+            _keep_selection(self.hadamard_bs, (n, sel))
             self._bs_tokens = key
         if input.is_cuda:
             n, sel = _selection(self.hadamard_bs)
