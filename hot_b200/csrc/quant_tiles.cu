@@ -3,7 +3,7 @@
 // A job is one tensor [batch, rows, channels] with a row side (Hadamard along the channels, codes as they lie: grad_output
 // for g_x), a column side (low-rank or Hadamard basis along the rows, codes transposed: grad_output for g_w, the weight, the
 // activation buffer), or both, and optionally the sum over all rows (the bias gradient).  Every CTA of either launch takes
-// one tile of one job: 64 channels (lane = a channel pair) by 128 or 256 rows, so that a small layer is two launches
+// one tile of one job: 64 channels (lane = a channel pair) by 64 to 256 rows, so that a small layer is two launches
 // instead of a clear, an abs-max and a quantise launch per operand, and a large one has thousands of equal tiles.
 //
 //   row side     a thread takes 16 channels of a row, straight from global memory (32- or 64-byte pieces, four lanes
