@@ -85,6 +85,7 @@ struct DevJobs {
   DevJob job[3];            // the main job, the weight, and another job of the main one's kind
   int third, sthird;        // first CTA of job[2], whose CTAs come after the main job's, in the second / first launch ...
   int first, sfirst;        // ... and of the weight, whose come last (beyond the grid: there is none)
+  int sums, sum_pairs;      // CTAs of the second launch that add up row sums, before all of these, and channel pairs of each
 };
 
 template <typename T>
@@ -738,33 +739,55 @@ __device__ __forceinline__ void quant_tile(const DevJob& j, int at, uint8_t* sme
       }
     }
   }
+  launch_dependents();
+}
 
-  if (!WEIGHT && j.part_sum && tile == 0 && b == 0) {  // the row sums of this channel block, partials in a fixed order
-    __syncthreads();
-    double* part = reinterpret_cast<double*>(smem);
-    const int c = threadIdx.x & 63, q = threadIdx.x >> 6, n = j.batch * j.stiles;
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    if (c0 + c < j.C) {
-      const float* p = j.part_sum + c0 + c;
-      for (int i = q; i < n; i += 8) {
+// The row sums of 2 * sum_pairs channels: the partials of every sample and tile, in a fixed order, eight loads of a thread in flight.
+// Few partials take all 64 channels of a block, many 16 (at the end of the first tiles' CTAs, half a channel's partials to a thread,
+// the sums were a tail: 32 x 784 x 128 in bf16 took both launches 26.9 us, now 14.1).
+constexpr int kManyPartials = 128;
+template <typename T>
+__device__ __forceinline__ void add_row_sums(const DevJob& j, int pairs, int block, uint8_t* smem) {
+  wait_for_predecessor();
+  double2* const part = reinterpret_cast<double2*>(smem);
+  const int lines = kThreads / pairs, pair = threadIdx.x % pairs, line = threadIdx.x / pairs, ch = 2 * (block * pairs + pair), n = j.batch * j.stiles;
+  double2 s = make_double2(0.0, 0.0);
+  if (ch < j.C) {
+    const float* p = j.part_sum + (int64_t)line * j.C + ch;
+    const int64_t step = (int64_t)lines * j.C;
+    for (int i = line; i < n; i += 8 * lines, p += 8 * step) {
+      float2 v[8];
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (i + 2 * k < n) s[k] += (double)__ldg(p + (int64_t)(i + 2 * k) * j.C);
+      for (int k = 0; k < 8; ++k) v[k] = i + k * lines < n ? __ldg(reinterpret_cast<const float2*>(p + k * step)) : make_float2(0.0f, 0.0f);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        s.x += (double)v[k].x;
+        s.y += (double)v[k].y;
       }
     }
-    part[threadIdx.x] = (s[0] + s[1]) + (s[2] + s[3]);
-    __syncthreads();
-    if (threadIdx.x < kCh && c0 + c < j.C) store_sum<T>(j.sum_out, c0 + c, (float)(part[c] + part[64 + c]));
+  }
+  part[threadIdx.x] = s;
+  __syncthreads();
+  const int c = 2 * block * pairs + (int)threadIdx.x;
+  if ((int)threadIdx.x < 2 * pairs && c < j.C) {
+    const double* q = reinterpret_cast<const double*>(part) + threadIdx.x;
+    double t = 0.0;
+    for (int k = 0; k < lines; ++k) t += q[k * 2 * pairs];
+    store_sum<T>(j.sum_out, c, (float)t);
   }
   launch_dependents();
 }
 
+// CTAs per SM: the registers that a loop without spills takes, but for bf16 where six with a few spills are faster (float32,
+// 6304 x 3072 and both other tensors of the extension call: 44.2 us for both launches with six, 42.5 with five).
 template <typename T, int MODE>
-__global__ void __launch_bounds__(kThreads, MODE == kColKept ? 5 : 6) tile_quant_kernel(const __grid_constant__ DevJobs jobs) {
+__global__ void __launch_bounds__(kThreads, MODE == kColKept || sizeof(T) == 4 ? 5 : 6) tile_quant_kernel(const __grid_constant__ DevJobs jobs) {
   extern __shared__ __align__(16) uint8_t smem[];  // kept rows as floats [position][64 channels]
-  if ((int)blockIdx.x < jobs.third) quant_tile<T, MODE, false>(jobs.job[0], blockIdx.x, smem);
-  else if ((int)blockIdx.x < jobs.first) quant_tile<T, MODE, false>(jobs.job[2], (int)blockIdx.x - jobs.third, smem);
-  else quant_tile<T, kColAll, true>(jobs.job[1], (int)blockIdx.x - jobs.first, smem);
+  const int cta = (int)blockIdx.x - jobs.sums;  // (the row sums' CTAs come first)
+  if (cta < 0) add_row_sums<T>(jobs.job[0], jobs.sum_pairs, blockIdx.x, smem);
+  else if (cta < jobs.third) quant_tile<T, MODE, false>(jobs.job[0], cta, smem);
+  else if (cta < jobs.first) quant_tile<T, MODE, false>(jobs.job[2], cta - jobs.third, smem);
+  else quant_tile<T, kColAll, true>(jobs.job[1], cta - jobs.first, smem);
 }
 
 // ---- host side --------------------------------------------------------------------------------------
@@ -920,7 +943,7 @@ int launch_tile_jobs(const TileJob* jobs, int count, int dtype, void* scratch, s
   memset(&dev, 0, sizeof(dev));
   dev.first = dev.sfirst = dev.third = dev.sthird = 1 << 30;
   int stats_ctas = 0, quant_ctas = 0;
-  size_t smem = kThreads * sizeof(double);
+  size_t smem = kThreads * sizeof(double2);
   uint8_t* at = (uint8_t*)scratch;
   for (int i : {0, 2, 1}) {
     if (i == 2 ? !third : i >= count) continue;
@@ -997,7 +1020,12 @@ int launch_tile_jobs(const TileJob* jobs, int count, int dtype, void* scratch, s
     if (i == 2) place_partials(t, g, (uint8_t*)third_scratch, &d);
     else at += place_partials(t, g, at, &d);
     d.sum_out = t.sum;
+    if (t.sum) {
+      dev.sum_pairs = t.batch * g.stiles > kManyPartials ? 8 : 32;
+      dev.sums = (int)((t.channels + 2 * dev.sum_pairs - 1) / (2 * dev.sum_pairs));
+    }
   }
+  quant_ctas += dev.sums;
   if (dtype == HOT_F32) return launch_typed<float>(dev, stats_ctas, quant_ctas, smem, st);
   return launch_typed<__nv_bfloat16>(dev, stats_ctas, quant_ctas, smem, st);
 }
