@@ -623,6 +623,26 @@ def test_row_ht_quant_pairs_of_runs(ops, rows, cols, order, lead, dtype, storage
     assert np.array_equal(_codes_from(codes, storage, cols), ref_c)
 
 
+@pytest.mark.parametrize("rows,cols,pad", [(1, 16, 0), (3, 48, 16), (7, 1024, 0), (5, 1040, 0), (600, 1056, 16), (1000, 1536, 0), (9, 8176, 0), (2, 8208, 0),
+                                           (450, 8192, 0), (3000, 96, 16), (4001, 80, 0)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("storage,bits,rounding", [("int4", 4, "philox"), ("int8", 8, "nearest")])
+@pytest.mark.parametrize("scale", ["tensor", "row"])
+def test_row_ht_quant_through_shared_memory(ops, rows, cols, pad, dtype, storage, bits, rounding, scale):
+    """Whole and ragged tiles of 1,024 elements, pitched rows, rows of whole warps that are no power of two, one and two pairs of runs
+    per thread, several turns of a persistent CTA: bit for bit the oracle's codes and scales."""
+    rng = np.random.default_rng(rows * 7 + cols)
+    x = (rng.standard_normal((rows, cols + pad)) * 1e-3).astype(np.float32)
+    x[:, cols:] = 7.0   # (beyond the row: must not be seen)
+    xd = _dev(x, dtype)[:, :cols]
+    codes, scales = ops.row_ht_quant(xd, 16, ops.Quant(bits, storage, rounding, scale, 11, 6))
+    xh = oc.fwht_last(_as_f32(x[:, :cols], dtype), 16)
+    u = _noise_for(rounding, (rows, cols), rng, 11, 6)
+    ref_c, ref_s = (oc.quant_rows if scale == "row" else oc.quant_tensor)(xh, bits, u)
+    assert np.array_equal(np.atleast_1d(ref_s).astype(np.float32).view(np.uint32), scales.cpu().numpy().view(np.uint32))
+    assert np.array_equal(_codes_from(codes, storage, cols), ref_c)
+
+
 def test_row_ht_quant_refuses_unknown_names(ops):
     x = torch.zeros((4, 64), device="cuda")
     for q in (ops.Quant(4, "int4", "nearest", "rows"), ops.Quant(4, "int4", "neareast", "row")):
