@@ -16,10 +16,10 @@
 // Every wait on an mbarrier is bounded in time; when a wait runs out the CTA ORs a code into
 // the caller's status word, stops issuing work, frees its tensor memory and returns.
 #include <cmath>
-#include <type_traits>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "tc.cuh"
@@ -1209,7 +1209,7 @@ int gemm_i8_dual_ws(const hot_gemm_problem_t* main_problem, const hot_gemm_probl
     int key[13];
     Plan s0, s1;
     int dual_bn, dual_split;
-    bool dual, dual_pair;
+    bool dual, dual_pair, swapped;
   };
   static std::mutex cache_mutex;
   static std::vector<Decision> cache;
@@ -1232,26 +1232,34 @@ int gemm_i8_dual_ws(const hot_gemm_problem_t* main_problem, const hot_gemm_probl
   if (!have) {
   const Plan s0 = make_plan(p0.M, p0.N, p0.num_kb, sms, 0, !a4, a4), s1 = make_plan(p1.M, p1.N, p1.num_kb, sms, 0, true, false);
   int dual_bn = 0, dual_split = 1;
-  bool dual_pair = false;
+  bool dual_pair = false, swapped = false;
   double together = 0.0;
   const int pair_mode = (e2 ? (e2[0] == '1' ? 2 : (e2[0] == '0' ? 0 : 1)) : 1);
+  for (const bool swap : {false, true})
   for (const bool pair : {false, true}) {
+    // Either problem may be the one of few, long tiles: with few tokens it is the first (49 x 768 over 3072 channels, 12 tiles of 24
+    // k-blocks beside 288 of one: 11.6 us in turn, 7.4 in one launch).
+    const GemmParams &q0 = swap ? p1 : p0, &q1 = swap ? p0 : p1;
+    if (swap && (a4 || force_split > 1 || q1.num_kb <= q0.num_kb)) continue;
     if (pair ? (pair_mode == 0 || a4 || sms < 2 || force_split > 1) : (pair_mode == 2 && !a4)) continue;
-    const int workers = pair ? sms / 2 : sms, tile_m = pair ? 2 * kBM : kBM;
-    for (int bn : {256, 192, 128}) {
-      if (bn == 128 && !pair) continue;
-      const int64_t t0 = (int64_t)((p0.M + tile_m - 1) / tile_m) * ((p0.N + bn - 1) / bn);
-      const int64_t t1 = (int64_t)((p1.M + tile_m - 1) / tile_m) * ((p1.N + bn - 1) / bn);
+    const int tile_m = pair ? 2 * kBM : kBM;
+    for (int bn : {256, 192, 128, 64}) {
+      if (bn <= 128 && a4) continue;
+      const int64_t t0 = (int64_t)((q0.M + tile_m - 1) / tile_m) * ((q0.N + bn - 1) / bn);
+      const int64_t t1 = (int64_t)((q1.M + tile_m - 1) / tile_m) * ((q1.N + bn - 1) / bn);
+      const int most = pair ? sms / 2 : sms, workers = (int)(t0 + t1 < most ? t0 + t1 : most);
       // (every worker holding a rider tile while the lag passes would leave nobody for the main tiles)
-      if (t1 > (pair ? workers - 1 : workers) || t0 < workers || t1 < 1) continue;
-      const double ns0 = tile_ns(p0.num_kb, bn, pair, a4);
+      if (t1 > (pair ? workers - 1 : workers) || (a4 && t0 < workers) || t0 < 1 || t1 < 1) continue;
+      // (tiles this narrow win only where there are few rounds of them; not replaying the others keeps a shape's first call short)
+      if (t0 > (bn == 64 ? 4 : 16) * (int64_t)workers && !(bn >= 192 || pair)) continue;
+      const double ns0 = tile_ns(q0.num_kb, bn, pair, a4);
       for (int split = 1; split <= 4; ++split) {
-        if (pair && split > 1) break;  // (the partial sums are parked per worker of one CTA)
+        if ((pair || swap) && split > 1) break;  // (the partial sums are parked per worker of one CTA)
         if (force_split > 0 ? split != force_split : split > 2) continue;  // more than two stretches only when asked (tests)
-        const int piece = (p1.num_kb + split - 1) / split;
+        const int piece = (q1.num_kb + split - 1) / split;
         if (split > 1) {
           // every stretch non-empty, a slot per worker with a stretch, a counter per rider tile
-          if (!workspace || !counters || t1 * split > sms || (int64_t)(split - 1) * piece >= p1.num_kb || t1 > 160 ||
+          if (!workspace || !counters || t0 < workers || t1 * split > sms || (int64_t)(split - 1) * piece >= q1.num_kb || t1 > 160 ||
               (size_t)(t1 * split) * kBM * bn * sizeof(int32_t) > workspace_bytes || ((uintptr_t)workspace) % 16 != 0)
             continue;
         }
@@ -1260,11 +1268,12 @@ int gemm_i8_dual_ws(const hot_gemm_problem_t* main_problem, const hot_gemm_probl
         // three or four (measured at ViT-B sizes: 768 x 768 x 6304 beside 12608 x 768 x 768 gains 2 us from
         // a cut in two and loses with three or four; larger riders lose with two).
         const double fix = split > 1 ? 8000.0 + 2300.0 * (split - 2) : 0.0;
-        const double c = launch_ns(bn, pair) + dual_max_load(t0, p0.num_kb, ns0, t1 * split, piece, tile_ns(piece, bn, pair, false), workers) + fix;
+        const double c = launch_ns(bn, pair) + dual_max_load(t0, q0.num_kb, ns0, t1 * split, piece, tile_ns(piece, bn, pair, false), workers) + fix;
         if (!dual_bn || c < together) {
           dual_bn = bn;
           dual_pair = pair;
           dual_split = split;
+          swapped = swap;
           together = c;
         }
       }
@@ -1278,6 +1287,7 @@ int gemm_i8_dual_ws(const hot_gemm_problem_t* main_problem, const hot_gemm_probl
     dec.dual_bn = dual_bn;
     dec.dual_split = dual_split;
     dec.dual_pair = dual_pair;
+    dec.swapped = swapped;
     dec.dual = dual;
     std::lock_guard<std::mutex> lock(cache_mutex);
     if (cache.size() >= 256) cache.clear();
@@ -1288,27 +1298,27 @@ int gemm_i8_dual_ws(const hot_gemm_problem_t* main_problem, const hot_gemm_probl
   const bool dual = dec.dual;
   if (dual) {
     if (dual_split > 1 && clear_words) HOT_CUDA(cudaMemsetAsync(counters, 0, clear_words * sizeof(uint32_t), st));
-    p1.split = dual_split;
-    p1.sk_partials = (int32_t*)workspace;
-    p1.sk_counters = counters;
-    Rider r{rider_problem->a, rider_problem->lda, rider_problem->b, rider_problem->ldb, p1};
-    const Plan plan{dual_bn, false, dec.dual_pair ? (unsigned)(sms / 2 * 2) : (unsigned)sms, dec.dual_pair};
-    const void* a = main_problem->a;
-    const void* b = main_problem->b;
-    const int64_t lda = main_problem->lda, ldb = main_problem->ldb;
-    if (dec.dual_pair) {
+    const hot_gemm_problem_t *first = dec.swapped ? rider_problem : main_problem, *second = dec.swapped ? main_problem : rider_problem;
+    GemmParams &q0 = dec.swapped ? p1 : p0, &q1 = dec.swapped ? p0 : p1;
+    q1.split = dual_split;
+    q1.sk_partials = (int32_t*)workspace;
+    q1.sk_counters = counters;
+    Rider r{second->a, second->lda, second->b, second->ldb, q1};
+    const int tile_m = dec.dual_pair ? 2 * kBM : kBM, most = dec.dual_pair ? sms / 2 : sms;
+    auto tiles = [&](const GemmParams& q) { return (int64_t)((q.M + tile_m - 1) / tile_m) * ((q.N + dual_bn - 1) / dual_bn); };
+    const int64_t all = tiles(q0) + tiles(q1) * dual_split, workers = all < most ? all : most;
+    const Plan plan{dual_bn, false, (unsigned)(dec.dual_pair ? 2 * workers : workers), dec.dual_pair};
+    auto launch = [&](auto packed, auto pair) -> int {
+      constexpr bool A4 = decltype(packed)::value, PAIR = decltype(pair)::value;
       switch (dual_bn) {
-        case 256: return launch_gemm<256, false, false, true>(a, lda, b, ldb, p0, plan, st, &r);
-        case 192: return launch_gemm<192, false, false, true>(a, lda, b, ldb, p0, plan, st, &r);
-        default: return launch_gemm<128, false, false, true>(a, lda, b, ldb, p0, plan, st, &r);
+        case 256: return launch_gemm<256, A4, false, PAIR>(first->a, first->lda, first->b, first->ldb, q0, plan, st, &r);
+        case 192: return launch_gemm<192, A4, false, PAIR>(first->a, first->lda, first->b, first->ldb, q0, plan, st, &r);
+        case 128: return launch_gemm<128, A4, false, PAIR>(first->a, first->lda, first->b, first->ldb, q0, plan, st, &r);
+        default: return launch_gemm<64, A4, false, PAIR>(first->a, first->lda, first->b, first->ldb, q0, plan, st, &r);
       }
-    }
-    if (dual_bn == 256) {
-      if (a4) return launch_gemm<256, true, false>(a, lda, b, ldb, p0, plan, st, &r);
-      return launch_gemm<256, false, false>(a, lda, b, ldb, p0, plan, st, &r);
-    }
-    if (a4) return launch_gemm<192, true, false>(a, lda, b, ldb, p0, plan, st, &r);
-    return launch_gemm<192, false, false>(a, lda, b, ldb, p0, plan, st, &r);
+    };
+    if (a4) return launch(std::true_type(), std::false_type());
+    return dec.dual_pair ? launch(std::false_type(), std::true_type()) : launch(std::false_type(), std::false_type());
   }
   int rc = a4 ? launch_bn<true, false>(main_problem->a, main_problem->lda, main_problem->b, main_problem->ldb, p0, s0, st)
               : launch_bn<false, false>(main_problem->a, main_problem->lda, main_problem->b, main_problem->ldb, p0, s0, st);

@@ -282,6 +282,23 @@ def _run_backward(ops, x, w, go, order_l, sel, dtype, *, gx_row=False, gw_row=Fa
     return gx, gw, ref
 
 
+@pytest.mark.parametrize("main_shape,rider_shape", [
+    ((49, 768, 3072), (3072, 768, 49)),          # few tokens: the first problem's tiles are the long ones
+    ((1, 16, 16), (16, 16, 16)),                 # one tile each
+    ((33, 4096, 4096), (4096, 4096, 33)),        # several rounds of short tiles beside them
+    ((300, 100, 256), (128, 128, 128)),          # ragged columns
+    ((130, 66, 1040), (1040, 66, 65)),           # two row tiles, outputs whose rows are not whole 16-byte pieces
+    ((2000, 1024, 1024), (1024, 1024, 1000)),
+])
+@pytest.mark.parametrize("pair", ["0", "1", None])
+def test_gemm_i8_dual_of_few_tokens(ops, main_shape, rider_shape, pair, monkeypatch):
+    """Either problem may ride, at every tile width and on single CTAs and pairs: bit for bit the separate products."""
+    if pair:
+        monkeypatch.setenv("HOT_GEMM_PAIR", pair)
+    monkeypatch.setenv("HOT_GEMM_DUAL", "1")
+    test_gemm_i8_dual(ops, main_shape, rider_shape, "int8", None, monkeypatch)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rounding", ["noise", "philox", "nearest"])
 @pytest.mark.parametrize("gx_row,gw_row", [(False, False), (True, True)])
