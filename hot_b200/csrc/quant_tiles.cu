@@ -85,7 +85,7 @@ struct DevJobs {
   DevJob job[3];            // the main job, the weight, and another job of the main one's kind
   int third, sthird;        // first CTA of job[2], whose CTAs come after the main job's, in the second / first launch ...
   int first, sfirst;        // ... and of the weight, whose come last (beyond the grid: there is none)
-  int sums, sum_pairs;      // CTAs of the second launch that add up row sums, before all of these, and channel pairs of each
+  int sums;                 // CTAs of the second launch that add up row sums, before all of these (0: the first tiles' do)
 };
 
 template <typename T>
@@ -582,7 +582,7 @@ __device__ __forceinline__ void row_side_any(const DevJob& j, const T* x, int b,
   }
 }
 
-template <typename T, int MODE, bool WEIGHT>
+template <typename T, int MODE, bool APART, bool WEIGHT>
 __device__ __forceinline__ void quant_tile(const DevJob& j, int at, uint8_t* smem) {
   __shared__ double s_mom[2][kWarps];
   const int rest = at / j.by_cblocks, cb = at - rest * j.cblocks;
@@ -739,18 +739,38 @@ __device__ __forceinline__ void quant_tile(const DevJob& j, int at, uint8_t* sme
       }
     }
   }
+
+  if (!WEIGHT && !APART && j.part_sum && tile == 0 && b == 0) {  // the row sums of this channel block, partials in a fixed order
+    __syncthreads();
+    double* part = reinterpret_cast<double*>(smem);
+    const int c = threadIdx.x & 63, q = threadIdx.x >> 6, n = j.batch * j.stiles;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    if (c0 + c < j.C) {
+      const float* p = j.part_sum + c0 + c;
+      for (int i = q; i < n; i += 8) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (i + 2 * k < n) s[k] += (double)__ldg(p + (int64_t)(i + 2 * k) * j.C);
+      }
+    }
+    part[threadIdx.x] = (s[0] + s[1]) + (s[2] + s[3]);
+    __syncthreads();
+    if (threadIdx.x < kCh && c0 + c < j.C) store_sum<T>(j.sum_out, c0 + c, (float)(part[c] + part[64 + c]));
+  }
   launch_dependents();
 }
 
-// The row sums of 2 * sum_pairs channels: the partials of every sample and tile, in a fixed order, eight loads of a thread in flight.
-// Few partials take all 64 channels of a block, many 16 (at the end of the first tiles' CTAs, half a channel's partials to a thread,
-// the sums were a tail: 32 x 784 x 128 in bf16 took both launches 26.9 us, now 14.1).
-constexpr int kManyPartials = 128;
+// Row sums of many partials (samples x tiles) come from CTAs of their own (APART): 16 channels each, the partials of every sample and
+// tile in a fixed order, eight loads of a thread in flight.  Summed by the CTAs of the first tiles, half a channel's partials to a thread,
+// they are a tail behind the codes: [32, 784, 128] in bf16, 416 partials, 26.9 us for both launches, 14.2 apart.  Few partials
+// stay there: [64, 197, 2304] and its 64 take 64.7 us, 65.7 apart.
+constexpr int kManyPartials = 128, kSumCh = 16;
 template <typename T>
-__device__ __forceinline__ void add_row_sums(const DevJob& j, int pairs, int block, uint8_t* smem) {
+__device__ __forceinline__ void add_row_sums(const DevJob& j, int block, uint8_t* smem) {
   wait_for_predecessor();
   double2* const part = reinterpret_cast<double2*>(smem);
-  const int lines = kThreads / pairs, pair = threadIdx.x % pairs, line = threadIdx.x / pairs, ch = 2 * (block * pairs + pair), n = j.batch * j.stiles;
+  constexpr int pairs = kSumCh / 2, lines = kThreads / pairs;
+  const int pair = threadIdx.x % pairs, line = threadIdx.x / pairs, ch = 2 * (block * pairs + pair), n = j.batch * j.stiles;
   double2 s = make_double2(0.0, 0.0);
   if (ch < j.C) {
     const float* p = j.part_sum + (int64_t)line * j.C + ch;
@@ -768,11 +788,12 @@ __device__ __forceinline__ void add_row_sums(const DevJob& j, int pairs, int blo
   }
   part[threadIdx.x] = s;
   __syncthreads();
-  const int c = 2 * block * pairs + (int)threadIdx.x;
-  if ((int)threadIdx.x < 2 * pairs && c < j.C) {
+  const int c = block * kSumCh + (int)threadIdx.x;
+  if ((int)threadIdx.x < kSumCh && c < j.C) {
     const double* q = reinterpret_cast<const double*>(part) + threadIdx.x;
     double t = 0.0;
-    for (int k = 0; k < lines; ++k) t += q[k * 2 * pairs];
+#pragma unroll
+    for (int k = 0; k < lines; ++k) t += q[k * kSumCh];
     store_sum<T>(j.sum_out, c, (float)t);
   }
   launch_dependents();
@@ -780,14 +801,16 @@ __device__ __forceinline__ void add_row_sums(const DevJob& j, int pairs, int blo
 
 // CTAs per SM: the registers that a loop without spills takes, but for bf16 where six with a few spills are faster (float32,
 // 6304 x 3072 and both other tensors of the extension call: 44.2 us for both launches with six, 42.5 with five).
-template <typename T, int MODE>
-__global__ void __launch_bounds__(kThreads, MODE == kColKept || sizeof(T) == 4 ? 5 : 6) tile_quant_kernel(const __grid_constant__ DevJobs jobs) {
+// CTAs per SM: the registers that a loop without spills takes where that is faster than six CTAs with a few spills (the extension call's
+// three float32 tensors of 6304 tokens: 44.0 us for both launches with six, 43.4 with five).
+template <typename T, int MODE, bool APART>
+__global__ void __launch_bounds__(kThreads, MODE == kColKept || (MODE == kColHalf16 && sizeof(T) == 4) ? 5 : 6) tile_quant_kernel(const __grid_constant__ DevJobs jobs) {
   extern __shared__ __align__(16) uint8_t smem[];  // kept rows as floats [position][64 channels]
-  const int cta = (int)blockIdx.x - jobs.sums;  // (the row sums' CTAs come first)
-  if (cta < 0) add_row_sums<T>(jobs.job[0], jobs.sum_pairs, blockIdx.x, smem);
-  else if (cta < jobs.third) quant_tile<T, MODE, false>(jobs.job[0], cta, smem);
-  else if (cta < jobs.first) quant_tile<T, MODE, false>(jobs.job[2], cta - jobs.third, smem);
-  else quant_tile<T, kColAll, true>(jobs.job[1], cta - jobs.first, smem);
+  const int cta = (int)blockIdx.x - (APART ? jobs.sums : 0);  // (the row sums' CTAs come first)
+  if (APART && cta < 0) add_row_sums<T>(jobs.job[0], blockIdx.x, smem);
+  else if (cta < jobs.third) quant_tile<T, MODE, APART, false>(jobs.job[0], cta, smem);
+  else if (cta < jobs.first) quant_tile<T, MODE, APART, false>(jobs.job[2], cta - jobs.third, smem);
+  else quant_tile<T, kColAll, APART, true>(jobs.job[1], cta - jobs.first, smem);
 }
 
 // ---- host side --------------------------------------------------------------------------------------
@@ -865,7 +888,8 @@ int launch_mode(const DevJobs& jobs, int stats_ctas, int quant_ctas, size_t smem
   const int dev = once.current(&done);
   if (dev < 0) HOT_FAIL(HOT_ERR_CUDA, "quant_tiles: cannot query the current CUDA device");
   if (!done) {
-    HOT_CUDA(cudaFuncSetAttribute(tile_quant_kernel<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 256 * kCh * (int)sizeof(float)));
+    for (auto kernel : {tile_quant_kernel<T, MODE, false>, tile_quant_kernel<T, MODE, true>})
+      HOT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 256 * kCh * (int)sizeof(float)));
     once.mark(dev);
   }
   // both may start while their predecessor on the stream drains; they wait for it before they touch memory
@@ -881,7 +905,7 @@ int launch_mode(const DevJobs& jobs, int stats_ctas, int quant_ctas, size_t smem
   HOT_CUDA(cudaLaunchKernelEx(&cfg, tile_stats_kernel<T, MODE>, jobs));
   cfg.gridDim = dim3((unsigned)quant_ctas);
   cfg.dynamicSmemBytes = smem;
-  HOT_CUDA(cudaLaunchKernelEx(&cfg, tile_quant_kernel<T, MODE>, jobs));
+  HOT_CUDA(cudaLaunchKernelEx(&cfg, jobs.sums ? tile_quant_kernel<T, MODE, true> : tile_quant_kernel<T, MODE, false>, jobs));
   return HOT_OK;
 }
 
@@ -1020,10 +1044,7 @@ int launch_tile_jobs(const TileJob* jobs, int count, int dtype, void* scratch, s
     if (i == 2) place_partials(t, g, (uint8_t*)third_scratch, &d);
     else at += place_partials(t, g, at, &d);
     d.sum_out = t.sum;
-    if (t.sum) {
-      dev.sum_pairs = t.batch * g.stiles > kManyPartials ? 8 : 32;
-      dev.sums = (int)((t.channels + 2 * dev.sum_pairs - 1) / (2 * dev.sum_pairs));
-    }
+    if (t.sum && t.batch * g.stiles > kManyPartials) dev.sums = (int)((t.channels + kSumCh - 1) / kSumCh);
   }
   quant_ctas += dev.sums;
   if (dtype == HOT_F32) return launch_typed<float>(dev, stats_ctas, quant_ctas, smem, st);
