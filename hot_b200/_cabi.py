@@ -105,6 +105,9 @@ EXPORTS = {
     "hot_layer_backward": (ctypes.c_int, [ctypes.POINTER(HotLayer), c_vp, c_vp, c_i64, c_vp, c_vp, c_vp, c_i64, c_vp, c_i64, c_vp, c_vp,
                                           ctypes.c_size_t, c_vp, c_vp]),
     "hot_im2col": (ctypes.c_int, [ctypes.POINTER(HotConv), c_vp, c_vp, c_vp]),
+    "hot_conv_folds": (ctypes.c_int, [ctypes.POINTER(HotLayer), ctypes.POINTER(HotConv)]),
+    "hot_layer_backward_conv": (ctypes.c_int, [ctypes.POINTER(HotLayer), ctypes.POINTER(HotConv), c_vp, c_vp, c_i64, c_vp, c_vp, c_vp, c_vp,
+                                               c_i64, c_vp, c_vp, ctypes.c_size_t, c_vp, c_vp]),
     "hot_col2im": (ctypes.c_int, [ctypes.POINTER(HotConv), c_vp, c_vp, c_vp]),
     "hot_transpose": (ctypes.c_int, [ctypes.c_int, c_i64, c_i64, c_i64, c_vp, c_vp, c_vp, c_vp]),
     "hot_add_bias": (ctypes.c_int, [c_vp, c_vp, c_i64, c_i64, c_vp]),

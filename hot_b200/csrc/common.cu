@@ -70,19 +70,12 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// Tensor map over a [rows, row_bytes] byte matrix with pitch ld, box = box_bytes x box_rows.
-}  // namespace
-
-int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t row_bytes, int64_t ld, int box_bytes,
-             int box_rows, int swizzle_bytes) {
+int encode_map(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box, int swizzle_bytes) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) HOT_FAIL(HOT_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-  cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)ld};
-  cuuint32_t box[2] = {(cuuint32_t)box_bytes, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
   auto encode = [&]() {
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, rank, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE),
                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   };
@@ -96,6 +89,27 @@ int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t row_bytes
   }
   if (r != CUDA_SUCCESS) HOT_FAIL(HOT_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
   return HOT_OK;
+}
+}  // namespace
+
+// Tensor map over a [rows, row_bytes] byte matrix with pitch ld, box = box_bytes x box_rows.
+int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t row_bytes, int64_t ld, int box_bytes,
+             int box_rows, int swizzle_bytes) {
+  const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)ld};
+  const cuuint32_t box[2] = {(cuuint32_t)box_bytes, (cuuint32_t)box_rows};
+  return encode_map(map, base, 2, dims, strides, box, swizzle_bytes);
+}
+
+int make_map_nd(CUtensorMap* map, const void* base, int rank, const int64_t* dims, const int64_t* strides, const int* box) {
+  cuuint64_t d[5], st[4];
+  cuuint32_t bx[5];
+  if (rank < 2 || rank > 5) HOT_FAIL(HOT_ERR_ARG, "tensor map of rank %d", rank);
+  for (int i = 0; i < rank; ++i) {
+    d[i] = (cuuint64_t)dims[i];
+    bx[i] = (cuuint32_t)box[i];
+    if (i + 1 < rank) st[i] = (cuuint64_t)strides[i];
+  }
+  return encode_map(map, base, rank, d, st, bx, 128);
 }
 
 

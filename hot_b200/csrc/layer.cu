@@ -197,7 +197,8 @@ int quantise_weight(const hot_layer_t& l, const Plan& p, const void* w, int64_t 
 
 int layer_backward(const hot_layer_t& l, const void* go, int64_t ldgo, const void* w, int64_t ldw, const void* x_q_t,
                    const float* scale_x, void* grad_x, int64_t ldgx, void* grad_w, int64_t ldgw, void* grad_b, void* workspace,
-                   size_t workspace_bytes, uint32_t* status, cudaEvent_t quantised, hot_stream_t stream, const CompressArgs* compress) {
+                   size_t workspace_bytes, uint32_t* status, cudaEvent_t quantised, hot_stream_t stream, const CompressArgs* compress,
+                   const hot_conv_t* fold) {
   if (!go || !w || !x_q_t || !scale_x || !workspace) HOT_FAIL(HOT_ERR_ARG, "hot_linear_backward: null pointer");
   if (!grad_x && !grad_w) HOT_FAIL(HOT_ERR_ARG, "hot_linear_backward: no output requested");
   if (int rc = check_layer(&l, "hot_linear_backward")) return rc;
@@ -289,6 +290,10 @@ int layer_backward(const hot_layer_t& l, const void* go, int64_t ldgo, const voi
 
   const float post_x = 1.0f / (float)c.order_o, post_w = 1.0f / (float)c.order_l;
   const int rows_per_scale = gx_row ? 1 : (l.batch ? (int)l.L : 0);
+  if (fold && grad_x) {
+    if (int rc = conv_grad_input(l, *fold, base + p.off_qgo, p.ld_qgo, s_go, base + p.off_qw, p.ld_qw, s_w, post_x, grad_x, status, st)) return rc;
+    grad_x = nullptr;
+  }
   if (l.batch) {
     if (grad_x)
       if (int rc = hot_gemm_i8(base + p.off_qgo, c.q_gx.storage, p.ld_qgo, base + p.off_qw, HOT_STORE_INT8, p.ld_qw, p.rows, l.I, l.O, s_go,
@@ -420,6 +425,16 @@ extern "C" int hot_layer_backward(const hot_layer_t* layer, const void* go, cons
   if (!layer) HOT_FAIL(HOT_ERR_ARG, "hot_layer_backward: null pointer");
   return layer_backward(*layer, go, layer->O, w, ldw, x_q_t, scale_x, grad_x, ldgx, grad_w, ldgw, grad_b, workspace, workspace_bytes,
                         status_word, nullptr, stream);
+}
+
+extern "C" int hot_layer_backward_conv(const hot_layer_t* layer, const hot_conv_t* conv, const void* go, const void* w, int64_t ldw,
+                                       const void* x_q_t, const float* scale_x, void* grad_x, void* grad_w, int64_t ldgw, void* grad_b,
+                                       void* workspace, size_t workspace_bytes, uint32_t* status_word, hot_stream_t stream) {
+  using namespace hot;
+  if (!layer || !conv) HOT_FAIL(HOT_ERR_ARG, "hot_layer_backward_conv: null pointer");
+  if (!conv_fold_covered(*layer, *conv)) HOT_FAIL(HOT_ERR_UNSUPPORTED, "hot_layer_backward_conv: not covered (see hot_conv_folds)");
+  return layer_backward(*layer, go, layer->O, w, ldw, x_q_t, scale_x, grad_x, layer->I, grad_w, ldgw, grad_b, workspace, workspace_bytes,
+                        status_word, nullptr, stream, nullptr, conv);
 }
 
 namespace hot {

@@ -29,11 +29,16 @@ struct CompressArgs {
   size_t workspace_bytes;
 };
 
-// The backward of one layer.  compress (nullable): the buffer (x_q_t, scale_x) is made first.  grad_b (nullable): the sum of go over its rows, in the tensors' type.  quantised
+// The input gradient of a convolution, folded by the product that makes it (gemm_conv.cu).
+bool conv_fold_covered(const hot_layer_t& layer, const hot_conv_t& conv);
+int conv_grad_input(const hot_layer_t& layer, const hot_conv_t& conv, const void* q_go, int64_t ld_go, const float* s_go, const void* q_w, int64_t ld_w,
+                    const float* s_w, float post, void* out, uint32_t* status, cudaStream_t st);
+
+// The backward of one layer.  fold (nullable): grad_x is that convolution's input gradient, not the rows'.  compress (nullable): the buffer (x_q_t, scale_x) is made first.  grad_b (nullable): the sum of go over its rows, in the tensors' type.  quantised
 // (nullable): an event recorded between the quantisers and the products.
 int layer_backward(const hot_layer_t& layer, const void* go, int64_t ldgo, const void* w, int64_t ldw, const void* x_q_t,
                    const float* scale_x, void* grad_x, int64_t ldgx, void* grad_w, int64_t ldgw, void* grad_b, void* workspace,
                    size_t workspace_bytes, uint32_t* status_word, cudaEvent_t quantised, hot_stream_t stream,
-                   const CompressArgs* compress = nullptr);
+                   const CompressArgs* compress = nullptr, const hot_conv_t* fold = nullptr);
 
 }  // namespace hot

@@ -11,6 +11,8 @@ namespace hot {
 // Tensor map over a [rows, row_bytes] byte matrix with pitch ld, box = box_bytes x box_rows.
 int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t row_bytes, int64_t ld, int box_bytes,
              int box_rows, int swizzle_bytes);  // swizzle_bytes: 0, 64 or 128
+// The same over `rank` dimensions of bytes (strides of all but the first), boxes swizzled by 128 bytes.
+int make_map_nd(CUtensorMap* map, const void* base, int rank, const int64_t* dims, const int64_t* strides, const int* box);
 
 // The time limit of every device-side wait: 1.5 s unless hot_set_wait_limit_ns changed it; the launchers copy it
 // into the kernel parameters (host side: common.cu).

@@ -235,9 +235,10 @@ struct Saved {
     for (int i = 0; i < c.rank_l; ++i) PyList_SetItem(sel, i, PyLong_FromLong(c.sel_l[i]));
     return Ref(Py_BuildValue("(LiiNii)", (long long)layer.batch, c.order_o, c.order_l, sel, c.q_x.bits, c.q_x.storage == HOT_STORE_INT4));
   }
-  // go: contiguous, w2: the weight as [O, I], both of one dtype; gx comes in the shape of go with I in place of O
+  // go: contiguous, w2: the weight as [O, I], both of one dtype; gx comes in the shape of go with I in place of O, or, for a
+  // convolution whose product folds it, as the image's gradient (folded is then set)
   void backward(const std::shared_ptr<Node>& node, const Tensor& go, const Tensor& w2, bool need_x, bool need_w, bool need_b, Tensor& gx,
-                Tensor& gw, Tensor& gb) const {
+                Tensor& gw, Tensor& gb, const hot_conv_t* conv = nullptr, bool* folded = nullptr) const {
     const Tensor codes = x_q_t.unpack(node), scale = scale_x.unpack(node);
     hot_layer_t l = layer;
     {
@@ -257,7 +258,11 @@ struct Saved {
     const size_t ws_bytes = hot_layer_backward_workspace_bytes(&l);
     if (ws_bytes == 0) fail(HOT_ERR_UNSUPPORTED, "hot_layer_backward");
     const Tensor ws = bytes((int64_t)ws_bytes, go);
-    if (need_x) {
+    const bool fold = need_x && conv && hot_conv_folds(&l, conv) != 0;
+    if (folded) *folded = fold;
+    if (fold) {
+      gx = at::empty({conv->B, conv->C, conv->H, conv->W}, go.options());
+    } else if (need_x) {
       std::vector<int64_t> shape = go.sizes().vec();
       shape.back() = l.I;
       gx = at::empty(shape, go.options());
@@ -270,6 +275,12 @@ struct Saved {
     // the bias gradient comes from the quantisers' own pass over grad_out where they can make it (they take channels in pairs)
     const bool sums = need_b && hot_layer_sums_rows(&l, go.data_ptr()) != 0;
     if (need_b) gb = sums ? at::empty({l.O}, go.options()) : go.reshape({-1, l.O}).sum(0);
+    if (fold)
+      check(hot_layer_backward_conv(&l, conv, go.data_ptr(), w2.data_ptr(), w2.stride(0), codes.data_ptr(), (const float*)scale.data_ptr(),
+                                    gx.data_ptr(), need_w ? gw.data_ptr() : nullptr, ldgw, sums ? gb.data_ptr() : nullptr, ws.data_ptr(), ws_bytes,
+                                    nullptr, current_stream()),
+            "hot_layer_backward_conv");
+    else
     check(hot_layer_backward(&l, go.data_ptr(), w2.data_ptr(), w2.stride(0), codes.data_ptr(), (const float*)scale.data_ptr(),
                              need_x ? gx.data_ptr() : nullptr, l.I, need_w ? gw.data_ptr() : nullptr, ldgw, sums ? gb.data_ptr() : nullptr,
                              ws.data_ptr(), ws_bytes, nullptr, current_stream()),
@@ -341,10 +352,13 @@ struct HotConvBackward : public Node {
     check(hot_transpose(conv.dtype, conv.B, s.layer.O, positions, go.data_ptr(), nullptr, rows.data_ptr(), current_stream()), "hot_transpose");
     Tensor gcols;
     Tensor gb;
-    s.backward(shared_from_this(), rows, w.view({s.layer.O, s.layer.I}), need_x, need_w, need_b, gcols, out[1], gb);
+    bool folded = false;
+    s.backward(shared_from_this(), rows, w.view({s.layer.O, s.layer.I}), need_x, need_w, need_b, gcols, out[1], gb, &conv, &folded);
     if (need_b) out[2] = gb;
     if (need_w) out[1] = out[1].reshape(w.sizes());  // (a copy where its rows are padded)
-    if (need_x) {
+    if (need_x && folded) {
+      out[0] = gcols;
+    } else if (need_x) {
       gcols = gcols.contiguous();
       out[0] = at::empty({conv.B, conv.C, conv.H, conv.W}, go.options());
       check(hot_col2im(&conv, gcols.data_ptr(), out[0].data_ptr(), current_stream()), "hot_col2im");

@@ -415,6 +415,13 @@ typedef struct hot_conv {
 } hot_conv_t;
 int hot_im2col(const hot_conv_t* conv, const void* x, void* cols, hot_stream_t stream);
 int hot_col2im(const hot_conv_t* conv, const void* cols, void* x, hot_stream_t stream);
+/* hot_layer_backward of a convolution whose rows are its output positions: grad_x is the input gradient [B, C, H, W] itself, folded by
+ * the product that makes it.  hot_conv_folds: whether (1 or 0) this layer and convolution are covered (stride 1, one scale per
+ * image or for all, one byte per g_x code); where they are not, hot_layer_backward makes the rows and hot_col2im folds them. */
+int hot_conv_folds(const hot_layer_t* layer, const hot_conv_t* conv);
+int hot_layer_backward_conv(const hot_layer_t* layer, const hot_conv_t* conv, const void* go, const void* w, int64_t ldw, const void* x_q_t,
+                            const float* scale_x, void* grad_x, void* grad_w, int64_t ldgw, void* grad_b, void* workspace,
+                            size_t workspace_bytes, uint32_t* status_word, hot_stream_t stream);
 int hot_transpose(int dtype, int64_t batch, int64_t rows, int64_t cols, const void* in, const void* bias, void* out,
                   hot_stream_t stream);
 int hot_add_bias(float* y, const float* bias, int64_t rows, int64_t cols, hot_stream_t stream);
