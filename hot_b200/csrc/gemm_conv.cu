@@ -3,13 +3,14 @@
 //
 // The product over unfolded rows writes kh * kw values per input element, which a fold then adds up.  All of them carry the same pair
 // of scales, so the sum may as well be the contraction: one integer product whose K runs over the taps too, and which leaves
-// nothing to fold.  A tile is 128 (or fewer) input positions of one image, whole rows where they fit, by up to 128 channels; for every tap
+// nothing to fold.  A tile is 128 (or fewer) input positions of one image, whole rows where they fit, by up to 256 channels; for every tap
 // the bulk copy fetches the grad_output rows of those positions moved by the tap, with zeros for what lies outside the image, and the kernel's
 // rows of that tap, c * kh * kw + tap, are a dimension of their tensor map.  The integer sums are exact and round once, where the taps
 // used to round one by one before they were added.
 //
-// What bounds it: the fill of shared memory (a stage of 32 KB per tap and 128 channels, about 200 ns), and for few channels the two trips
-// to start and to drain.  32 x 128 x 28 x 28, 3 x 3, 128 outputs, bf16: @CONV@.
+// What bounds it: the fill of shared memory (32 to 48 KB per tap and 128 outputs, 200 to 330 ns), and for few channels the start and
+// the drain.  32 x 128 x 28 x 28, 3 x 3, 128 outputs, bf16: 15 us, where the product over unfolded rows and the fold took 19 and 27; tiles
+// of 128 channels at most made the step of 64 x 256 x 56 x 56 to 512, 1 x 1, 1223 us, 256 make it 1209 (1213 with product and fold).
 #include <cstring>
 
 #include "layer.cuh"
@@ -21,8 +22,8 @@ int device_sm_count();
 
 namespace {
 
-constexpr int kBM = 128, kBK = 128, kMaxBN = 128;
-constexpr int kStages = 6, kStageA = kBM * kBK, kStageB = kMaxBN * kBK;
+constexpr int kBM = 128, kBK = 128, kMaxBN = 256;
+constexpr int kStages = 4, kStageA = kBM * kBK, kStageB = kMaxBN * kBK;
 constexpr int kEpiWarps = 8, kThreads = (kEpiWarps + 2) * 32;
 constexpr int kOffB = kStages * kStageA, kOffBar = kOffB + kStages * kStageB;
 constexpr int kSmem = kOffBar + 256 + 1024;
@@ -247,7 +248,7 @@ int conv_grad_input(const hot_layer_t& l, const hot_conv_t& v, const void* q_go,
   p.th = (p.H + rows - 1) / rows;
   p.bh = (p.H + p.th - 1) / p.th;
   p.tw = (p.W + p.bw - 1) / p.bw;
-  // channels: 128, fewer where that leaves SMs idle
+  // channels: up to 256, fewer where that leaves SMs idle
   const int64_t m_tiles = (int64_t)v.B * p.th * p.tw;
   p.bn = p.C >= kMaxBN ? kMaxBN : (p.C + 31) / 32 * 32;
   while (p.bn > 32 && m_tiles * ((p.C + p.bn - 1) / p.bn) < sms) p.bn = (p.bn / 2 + 31) / 32 * 32;
