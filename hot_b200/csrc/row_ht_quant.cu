@@ -249,9 +249,10 @@ __device__ __forceinline__ void store_run(uint8_t* dst, const uint32_t (&w)[4]) 
 // ---------------------------------------------------------------------------------------
 // per-row scale: one pass, row resident in registers
 // ---------------------------------------------------------------------------------------
-// Two kernels.  Rows of 4-byte elements come through shared memory, to persistent CTAs; rows of 2-byte elements straight from global
-// memory, a CTA for each row or few: those are bound by issue, and the copies only added to it (us, direct / staged: 16384 x 4096 bf16
-// 47.3 / 47.2, 58932 x 384 22.7 / 25.1, 32768 x 8192 213 / 217; float32 6304 x 3072 22.7 / 20.6, 65536 x 1024 68.7 / 57.5).
+// Two kernels.  Rows of 4-byte elements come through shared memory, to persistent CTAs; rows of 2-byte elements, and short ones, straight
+// from global memory, a CTA for each row or few: those are bound by issue, and the copies only added to it (us, direct / staged:
+// 16384 x 4096 bf16 47.3 / 47.2, 58932 x 384 22.7 / 25.1, 32768 x 8192 213 / 217; float32 6304 x 3072 22.7 / 20.6, 65536 x 1024
+// 68.7 / 57.5, 12608 x 512 12.0 / 10.4, 10705 x 256 6.3 / 8.3).
 //
 // kPairs: pairs of runs per thread (1 or 2).  tpr, the threads of a row: the power of two that gives each one pair, from 4 to
 // the CTA: short rows share a warp.
@@ -589,38 +590,43 @@ int launch_typed(const T* x, int64_t rows, int cols, int64_t ldx, int n, const h
   const QuantDev q = make_quant_dev(hq);
   if (hq.scale_mode == HOT_SCALE_ROW) {
     const int npair = ((cols >> 4) + 1) / 2;
-    constexpr bool kStaged = sizeof(T) == 4;
+    const bool staged = sizeof(T) == 4 && npair >= 16;
     int tpr = 4;
-    while (tpr < (kStaged ? 32 : kThreads) && tpr < npair) tpr <<= 1;  // one pair per thread while a CTA can hold the row
-    if (kStaged && npair > 32) tpr = npair >= kThreads ? kThreads : (npair + 31) / 32 * 32;
+    while (tpr < (staged ? 32 : kThreads) && tpr < npair) tpr <<= 1;  // one pair per thread while a CTA can hold the row
+    if (staged && npair > 32) tpr = npair >= kThreads ? kThreads : (npair + 31) / 32 * 32;
     if (npair > kMaxPairs * tpr)
       HOT_FAIL(HOT_ERR_UNSUPPORTED, "hot_row_ht_quant: per-row scale supports cols <= %d (got %d)", kMaxPairs * 32 * kThreads, cols);
     const int rows_per_cta = kThreads / tpr;
     const int64_t groups = (rows + rows_per_cta - 1) / rows_per_cta;
-    if constexpr (kStaged) {
-      auto run = [&](auto kernel, int pairs, PerDeviceOnce& once) -> int {
-        const int warp_bytes = pairs * WarpTile<T>::kBytes, threads = rows_per_cta * tpr;
-        if (int rc = allow_smem(kernel, kThreads / 32 * warp_bytes, once)) return rc;
-        const int64_t most = (int64_t)sms * (pairs == 1 ? 3 * kThreads / threads : 1);
-        kernel<<<(unsigned)(groups < most ? groups : most), threads, threads / 32 * warp_bytes, st>>>(x, rows, cols, ldx, n, q, codes, ld_codes, scales, tpr,
-                                                                                                      rows_per_cta);
-        return HOT_OK;
-      };
-      static PerDeviceOnce once2, once16, once32, once64, once0;
-      const int rc = npair > tpr ? run(row_ht_quant_rowscale_staged_kernel<T, ROUND, STORE4, 2, 0>, 2, once2)
-                     : n == 16   ? run(row_ht_quant_rowscale_staged_kernel<T, ROUND, STORE4, 1, 16>, 1, once16)
-                     : n == 32   ? run(row_ht_quant_rowscale_staged_kernel<T, ROUND, STORE4, 1, 32>, 1, once32)
-                     : n == 64   ? run(row_ht_quant_rowscale_staged_kernel<T, ROUND, STORE4, 1, 64>, 1, once64)
-                                 : run(row_ht_quant_rowscale_staged_kernel<T, ROUND, STORE4, 1, 0>, 1, once0);
-      if (rc) return rc;
-    } else {
-      const bool wide = (uintptr_t)x % 32 == 0 && ldx * sizeof(T) % 32 == 0;
-      auto kernel = npair > tpr ? row_ht_quant_rowscale_kernel<T, ROUND, STORE4, 2, 0>
-                    : n == 16   ? row_ht_quant_rowscale_kernel<T, ROUND, STORE4, 1, 16>
-                    : n == 32   ? row_ht_quant_rowscale_kernel<T, ROUND, STORE4, 1, 32>
-                    : n == 64   ? row_ht_quant_rowscale_kernel<T, ROUND, STORE4, 1, 64>
-                                : row_ht_quant_rowscale_kernel<T, ROUND, STORE4, 1, 0>;
-      kernel<<<(unsigned)groups, kThreads, 0, st>>>(x, rows, cols, ldx, n, q, codes, ld_codes, scales, tpr, wide);
+    if constexpr (sizeof(T) == 4) {
+      if (staged) {
+        auto run = [&](auto kernel, int pairs, PerDeviceOnce& once) -> int {
+          const int warp_bytes = pairs * WarpTile<T>::kBytes, threads = rows_per_cta * tpr;
+          if (int rc = allow_smem(kernel, kThreads / 32 * warp_bytes, once)) return rc;
+          const int64_t most = (int64_t)sms * (pairs == 1 ? 3 * kThreads / threads : 1);
+          kernel<<<(unsigned)(groups < most ? groups : most), threads, threads / 32 * warp_bytes, st>>>(x, rows, cols, ldx, n, q, codes, ld_codes, scales, tpr,
+                                                                                                        rows_per_cta);
+          HOT_CUDA(cudaGetLastError());
+          return HOT_OK;
+        };
+        static PerDeviceOnce once2, once16, once32, once64, once0;
+        return npair > tpr ? run(row_ht_quant_rowscale_staged_kernel<T, ROUND, STORE4, 2, 0>, 2, once2)
+               : n == 16   ? run(row_ht_quant_rowscale_staged_kernel<T, ROUND, STORE4, 1, 16>, 1, once16)
+               : n == 32   ? run(row_ht_quant_rowscale_staged_kernel<T, ROUND, STORE4, 1, 32>, 1, once32)
+               : n == 64   ? run(row_ht_quant_rowscale_staged_kernel<T, ROUND, STORE4, 1, 64>, 1, once64)
+                           : run(row_ht_quant_rowscale_staged_kernel<T, ROUND, STORE4, 1, 0>, 1, once0);
+      }
+    }
+    const bool wide = (uintptr_t)x % 32 == 0 && ldx * sizeof(T) % 32 == 0;
+    auto direct = [&](auto kernel) { kernel<<<(unsigned)groups, kThreads, 0, st>>>(x, rows, cols, ldx, n, q, codes, ld_codes, scales, tpr, wide); };
+    if constexpr (sizeof(T) == 2) {  // (4-byte rows this long are staged)
+      if (npair > tpr) direct(row_ht_quant_rowscale_kernel<T, ROUND, STORE4, 2, 0>);
+    }
+    if (npair <= tpr) {
+      if (n == 16) direct(row_ht_quant_rowscale_kernel<T, ROUND, STORE4, 1, 16>);
+      else if (n == 32) direct(row_ht_quant_rowscale_kernel<T, ROUND, STORE4, 1, 32>);
+      else if (n == 64) direct(row_ht_quant_rowscale_kernel<T, ROUND, STORE4, 1, 64>);
+      else direct(row_ht_quant_rowscale_kernel<T, ROUND, STORE4, 1, 0>);
     }
   } else {
     const Runs t = {rows * (cols >> 4), ldx, ld_codes, cols >> 4, ldx == cols && ld_codes == (STORE4 ? cols / 2 : cols),
