@@ -222,6 +222,9 @@ __global__ void __launch_bounds__(kThreads, 1)
 // hold.  (A dilation wider than the output leaves positions that no tap reaches, which have to be 0 whatever the scales.)
 bool conv_fold_covered(const hot_layer_t& l, const hot_conv_t& v) {
   const hot_linear_cfg_t& c = l.cfg;
+  if (v.B <= 0 || v.C <= 0 || v.H <= 0 || v.W <= 0 || v.kh <= 0 || v.kw <= 0 || v.dh <= 0 || v.dw <= 0 || v.ph < 0 || v.pw < 0 || v.dtype != c.dtype ||
+      l.O <= 0 || c.q_w.bits < 2 || c.q_w.bits > 8)
+    return false;
   if (v.sh != 1 || v.sw != 1 || c.q_gx.scale_mode != HOT_SCALE_TENSOR || c.q_gx.storage != HOT_STORE_INT8) return false;
   const int64_t oh = v.H + 2 * v.ph - (int64_t)v.dh * (v.kh - 1), ow = v.W + 2 * v.pw - (int64_t)v.dw * (v.kw - 1);
   if (oh < v.dh || ow < v.dw || oh > (1 << 20) || ow > (1 << 20) || v.H > (1 << 20) || v.W > (1 << 20) || v.C > (1 << 20) || v.B > 65535) return false;

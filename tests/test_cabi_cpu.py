@@ -129,3 +129,25 @@ def test_kept_selection_of_a_matrix_that_comes_to_lie_where_another_did():
         assert list(_selection(m)[1]) == rows.tolist() and list(_selection(m)[1]) == rows.tolist()
         m.copy_(torch.tensor(hadamard(16)[rows[::-1].copy()]))
         assert list(_selection(m)[1]) == rows[::-1].tolist()
+
+
+@pytest.mark.parametrize("change,covered", [
+    ({}, 1), ({"sh": 2}, 0), ({"sw": 2}, 0), ({"kh": 0}, 0), ({"ph": -1}, 0), ({"dtype": 1}, 0), ({"dh": 40}, 0), ({"H": 15}, 0),
+    ({"scale_mode": 1}, 0), ({"storage": 1}, 0), ({"w_bits": 9}, 0), ({"w_bits": 8}, 1), ({"O": 1 << 20, "w_bits": 8}, 0), ({"batch": 3}, 0),
+])
+def test_which_convolutions_fold_their_own_gradient(cabi, change, covered):
+    """Stride 1, one scale per image, one byte per code, positions that agree with the layer's, every position within reach of a tap, and
+    sums that 32 bits hold."""
+    lib = cabi.lib()
+    v = cabi.HotConv(0, 2, 8, 16, 16, 3, 3, 1, 1, 1, 1, 1, 1)
+    for k in ("sh", "sw", "kh", "ph", "dtype", "dh", "H"):
+        if k in change:
+            setattr(v, k, change[k])
+    cfg = cabi.HotLinearCfg()
+    cfg.order_o, cfg.order_l, cfg.rank_l = 16, 1, 1
+    for q in (cfg.q_gx, cfg.q_w, cfg.q_gw, cfg.q_x):
+        q.bits = 4
+    cfg.q_gx.scale_mode, cfg.q_gx.storage, cfg.q_w.bits = change.get("scale_mode", 0), change.get("storage", 0), change.get("w_bits", 4)
+    layer = cabi.HotLayer(change.get("batch", 2), 256, change.get("O", 32), 72, cfg)
+    assert lib.hot_conv_folds(ctypes.byref(layer), ctypes.byref(v)) == covered
+    assert lib.hot_conv_folds(None, ctypes.byref(v)) == 0
