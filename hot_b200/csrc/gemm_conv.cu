@@ -1,16 +1,18 @@
 // Input gradient of a convolution of stride 1 from the codes of grad_output and of the kernel, folded as it is made:
-//   grad_x[b, c, h, w] = (sum over taps (i, j) and channels o of  q_go[b, h + ph - i dh, w + pw - j dw, o] * q_w[c, (i, j), o]) * s_go[b] * s_w * post
+//   grad_x[b, c, h, w] = sum over taps (i, j) of round(s_go[b] * s_w * post * sum over o of  q_go[b, h + ph - i dh, w + pw - j dw, o] * q_w[c, (i, j), o])
 //
-// The product over unfolded rows writes kh * kw values per input element, which a fold then adds up.  All of them carry the same pair
-// of scales, so the sum may as well be the contraction: one integer product whose K runs over the taps too, and which leaves
-// nothing to fold.  A tile is 128 (or fewer) input positions of one image, whole rows where they fit, by up to 256 channels; for every tap
-// the bulk copy fetches the grad_output rows of those positions moved by the tap, with zeros for what lies outside the image, and the kernel's
-// rows of that tap, c * kh * kw + tap, are a dimension of their tensor map.  The integer sums are exact and round once, where the taps
-// used to round one by one before they were added.
+// The product over unfolded rows writes kh * kw values per input element, which a fold then reads and adds up.  Here a tile is 128 (or
+// fewer) input positions of one image, whole rows where they fit, by up to 128 channels; for every tap the bulk copy fetches the
+// grad_output rows of those positions moved by the tap, with zeros for what lies outside the image, and the kernel's rows of that tap,
+// c * kh * kw + tap, are a dimension of their tensor map.  A tap's integer sums are complete in a tensor-memory buffer of their own; the
+// epilogue scales and rounds them to the tensors' type as the product over rows would and adds them to its registers in the fold's order, so
+// that the result is, bit for bit, what product and fold give (also for scales and gradients that overflow or are infinite): which way a
+// size goes, or whether a layer runs natively, changes no value.  Convolutions of one tap keep no sums and take up to 256 channels.
 //
-// What bounds it: the fill of shared memory (32 to 48 KB per tap and 128 outputs, 200 to 330 ns), and for few channels the start and
-// the drain.  32 x 128 x 28 x 28, 3 x 3, 128 outputs, bf16: 15 us, where the product over unfolded rows and the fold took 19 and 27; tiles
-// of 128 channels at most made the step of 64 x 256 x 56 x 56 to 512, 1 x 1, 1223 us, 256 make it 1209 (1213 with product and fold).
+// What bounds it: the epilogue (five instructions a value and tap and the conversions; some 600 ns for a tap of 128 x 128), then the fill of
+// shared memory (32 KB per tap and 128 outputs, 250 to 330 ns). 32 x 128 x 28 x 28, 3 x 3, 128 outputs, bf16: the whole training step 159 us, 202
+// with product and fold; sixteen warps in the epilogue, or integers converted by an addition, were 1 to 6 % slower. (Summing the taps
+// as integers, rounded once, takes 154 and gives other values.)
 #include <cstring>
 
 #include "layer.cuh"
@@ -22,19 +24,26 @@ int device_sm_count();
 
 namespace {
 
-constexpr int kBM = 128, kBK = 128, kMaxBN = 256;
-constexpr int kStages = 4, kStageA = kBM * kBK, kStageB = kMaxBN * kBK;
-constexpr int kEpiWarps = 8, kThreads = (kEpiWarps + 2) * 32;
-constexpr int kOffB = kStages * kStageA, kOffBar = kOffB + kStages * kStageB;
-constexpr int kSmem = kOffBar + 256 + 1024;
-constexpr uint32_t kTmemCols = 2 * kMaxBN;
+constexpr int kBM = 128, kBK = 128;
+constexpr int kEpiWarps = 8, kTeams = kEpiWarps / 4, kThreads = (kEpiWarps + 2) * 32;
+constexpr uint32_t kTmemCols = 512;
+
+// ONE: convolutions of one tap
+template <bool ONE>
+struct Layout {
+  static constexpr int kMaxBN = ONE ? 256 : 128;
+  static constexpr int kBufs = (int)kTmemCols / kMaxBN;  // accumulators in tensor memory
+  static constexpr int kStageA = kBM * kBK, kStageB = kMaxBN * kBK, kStages = ONE ? 4 : 6;
+  static constexpr int kOffB = kStages * kStageA, kOffBar = kOffB + kStages * kStageB;
+  static constexpr int kSmem = kOffBar + 256 + 1024;
+};
 
 struct FoldParams {
   int H, W, C;
   int bw, bh;               // positions of a tile: bw columns of bh rows
   int tw, th;               // tiles across an image, and down
   int n_tiles, num_tiles, bn;
-  int kh, kw, dh, dw, ph, pw;
+  int OH, OW, kh, kw, dh, dw, ph, pw;
   int kblocks, last_steps;  // k-blocks of a tap; instructions of 32 in the last of them
   FastDiv by_n, by_tw, by_th, by_bw;
   uint32_t tx;              // bytes of a stage
@@ -42,8 +51,9 @@ struct FoldParams {
   int sa_batch;             // one scale per image
   const float* sb;
   float post;
+  int lean;                 // post goes with sb, as in the product over rows whose output begins on 16-byte pieces
+  float one;                // 1, in a place where the compiler does not see it
   void* out;
-  int out16;
   uint32_t* status;
   uint64_t wait_ns;
 };
@@ -70,15 +80,18 @@ struct FoldTile {
   }
 };
 
+template <bool ONE, bool OUT16>
 __global__ void __launch_bounds__(kThreads, 1)
     conv_fold_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const __grid_constant__ FoldParams p) {
+  using L = Layout<ONE>;
+  constexpr int kStages = L::kStages, kStageA = L::kStageA, kStageB = L::kStageB, kOffB = L::kOffB, kBufs = L::kBufs;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kOffBar);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::kOffBar);
   uint64_t* empty = full + kStages;
-  uint64_t* tmem_full = empty + kStages;  // [2] a tile's accumulator is complete
-  uint64_t* tmem_empty = tmem_full + 2;   // [2] drained
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+  uint64_t* tmem_full = empty + kStages;     // [kBufs] a tap's sums are complete
+  uint64_t* tmem_empty = tmem_full + kBufs;  // [kBufs] drained
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + kBufs);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int kProducer = kEpiWarps, kMma = kProducer + 1;
@@ -88,7 +101,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < kBufs; ++b) {
       mbar_init(&tmem_full[b], 1);
       mbar_init(&tmem_empty[b], kEpiWarps);
     }
@@ -112,8 +125,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       bool ok = true;
       for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
         const FoldTile t(p, tile);
-        int i = 0, j = 0;
-        for (int tap = 0; ok && tap < taps; ++tap) {
+        int i = p.kh - 1, j = p.kw - 1;  // (the fold adds ascending output positions)
+        for (int tap = taps - 1; ok && tap >= 0; --tap) {
           for (int kb = 0; kb < p.kblocks; ++kb, s = (s + 1 == kStages ? 0 : s + 1), ph ^= (s == 0 ? 1u : 0u)) {
             ok = mbar_wait(&empty[s], ph ^ 1u, abort_flag, p.wait_ns);
             if (!ok) break;
@@ -121,9 +134,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             tma_load_4d(smem + s * kStageA, &tma_a, &full[s], kb * kBK, t.w0 + p.pw - j * p.dw, t.h0 + p.ph - i * p.dh, t.b);
             tma_load_3d(smem + kOffB + s * kStageB, &tma_b, &full[s], kb * kBK, tap, t.n0);
           }
-          if (++j == p.kw) {
-            j = 0;
-            ++i;
+          if (--j < 0) {
+            j = p.kw - 1;
+            --i;
           }
         }
       }
@@ -135,14 +148,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t a_lo0 = (uint32_t)smem_desc_sw128(smem_u32(smem)), b_lo0 = (uint32_t)smem_desc_sw128(smem_u32(smem + kOffB));
       uint32_t s = 0, ph = 0, it = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x, ++it) {
-        const uint32_t buf = it & 1u, bph = (it >> 1) & 1u;
-        ok = mbar_wait(&tmem_empty[buf], bph ^ 1u, abort_flag, p.wait_ns);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t d = tmem_base + buf * kMaxBN;
-        uint32_t accumulate = 0u;
-        for (int tap = 0; ok && tap < taps; ++tap)
+      for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x)
+        for (int tap = 0; ok && tap < taps; ++tap, ++it) {
+          const uint32_t buf = it % kBufs, bph = (it / kBufs) & 1u;
+          ok = mbar_wait(&tmem_empty[buf], bph ^ 1u, abort_flag, p.wait_ns);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t d = tmem_base + buf * L::kMaxBN;
           for (int kb = 0; kb < p.kblocks; ++kb, s = (s + 1 == kStages ? 0 : s + 1), ph ^= (s == 0 ? 1u : 0u)) {
             ok = mbar_wait(&full[s], ph, abort_flag, p.wait_ns);
             if (!ok) break;
@@ -151,53 +163,100 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int steps = kb + 1 == p.kblocks ? p.last_steps : kBK / 32;
 #pragma unroll
             for (int k = 0; k < kBK / 32; ++k)
-              if (k < steps) {
-                umma_i8(d, ((uint64_t)hi << 32) | (a_lo + 2u * k), ((uint64_t)hi << 32) | (b_lo + 2u * k), idesc, accumulate);
-                accumulate = 1u;
-              }
+              if (k < steps) umma_i8(d, ((uint64_t)hi << 32) | (a_lo + 2u * k), ((uint64_t)hi << 32) | (b_lo + 2u * k), idesc, kb > 0 || k > 0 ? 1u : 0u);
             umma_commit(&empty[s]);
           }
-        if (ok) umma_commit(&tmem_full[buf]);
-      }
+          if (ok) umma_commit(&tmem_full[buf]);
+        }
     }
   } else {
-    const int q = warp & 3, team = warp >> 2;  // tensor-memory lane quarter; of the chunks of 32 channels, the even or the odd ones
+    const int q = warp & 3, team = warp >> 2;  // tensor-memory lane quarter; share of the tile's columns
     const int m = q * 32 + lane, hh = m / p.by_bw, ww = m - hh * p.bw;
-    const int chunks = p.bn / 32;
+    const int per = (p.bn / 32 + kTeams - 1) / kTeams, first = team * per, mine = min(per, p.bn / 32 - first);  // this warp's chunks of 32 channels
+    constexpr int kChunks = L::kMaxBN / (32 * kTeams), kSums = ONE ? 1 : kChunks;
     const int64_t plane = (int64_t)p.H * p.W;
-    const float sb = __ldg(p.sb);
+    const float sb = __ldg(p.sb), fb = p.lean ? __fmul_rn(sb, p.post) : sb;
+    const float2 post2 = make_float2(p.post, p.post), one2 = make_float2(p.one, p.one);
     uint32_t it = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x, ++it) {
+    for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
       const FoldTile t(p, tile);
-      const uint32_t buf = it & 1u, bph = (it >> 1) & 1u;
+      const int h = t.h0 + hh, w = t.w0 + ww;
       const float sa = __ldg(p.sa + (p.sa_batch ? t.b : 0));
-      ok = __all_sync(0xFFFFFFFFu, mbar_wait_parked(&tmem_full[buf], bph, abort_flag, p.wait_ns)) != 0;
-      if (!ok) break;
-      tc_fence_after();
-      const bool inside = hh < p.bh && t.h0 + hh < p.H && t.w0 + ww < p.W;
-      const int64_t at = ((int64_t)t.b * p.C + t.n0) * plane + (int64_t)(t.h0 + hh) * p.W + t.w0 + ww;
-      for (int c = team; c < chunks; c += 2) {
-        uint32_t acc[32];
-        tmem_ld32(tmem_base + buf * kMaxBN + ((uint32_t)(q * 32) << 16) + c * 32, acc);
-        if (!inside) continue;
+      const bool inside = hh < p.bh && h < p.H && w < p.W;
+      const int64_t at = ((int64_t)t.b * p.C + t.n0) * plane + (int64_t)h * p.W + w;
+      float2 sum[kSums][16];
+      auto open = [&](float2 (&v)[16]) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = make_float2(0.0f, 0.0f);
+      };
+      // one tap of 32 channels: scaled and rounded as the product over rows stores it, then added.  (A tap outside the output has sums of
+      // zero and comes with scales of zero: it adds nothing.)
+      auto add = [&](float2 (&v)[16], const uint32_t (&acc)[32], float ta, float tb) {
+        const float2 fa2 = make_float2(ta, ta), fb2 = make_float2(tb, tb);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          float2 f = __fmul2_rn(__fmul2_rn(make_float2((float)(int)acc[2 * i], (float)(int)acc[2 * i + 1]), fa2), fb2);
+          if (!p.lean) f = __fmul2_rn(f, post2);
+          if (OUT16) {
+            const __nv_bfloat162 r = __floats2bfloat162_rn(f.x, f.y);
+            const uint32_t bits = *reinterpret_cast<const uint32_t*>(&r);
+            v[i] = add2(v[i], make_float2(__uint_as_float(bits << 16), __uint_as_float(bits & 0xFFFF0000u)));
+          } else {
+            v[i] = __ffma2_rn(f, one2, v[i]);  // (as an addition it would be joined with the product before it)
+          }
+        }
+      };
+      auto store = [&](const float2 (&v)[16], int c) {
         const int left = p.C - t.n0 - c * 32;  // channels from this chunk on
-        auto value = [&](int i) { return __fmul_rn(__fmul_rn(__fmul_rn((float)(int)acc[i], sa), sb), p.post); };
-        if (p.out16) {
+        if (OUT16) {
           __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + at + (int64_t)(c * 32) * plane;
 #pragma unroll
           for (int i = 0; i < 32; ++i, o += plane)
-            if (i < left) *o = __float2bfloat16_rn(value(i));
+            if (i < left) *o = __float2bfloat16_rn(i & 1 ? v[i / 2].y : v[i / 2].x);
         } else {
           float* o = reinterpret_cast<float*>(p.out) + at + (int64_t)(c * 32) * plane;
 #pragma unroll
           for (int i = 0; i < 32; ++i, o += plane)
-            if (i < left) *o = value(i);
+            if (i < left) *o = i & 1 ? v[i / 2].y : v[i / 2].x;
+        }
+      };
+      if (!ONE)
+#pragma unroll
+        for (int k = 0; k < kSums; ++k) open(sum[k]);
+      int oh = h + p.ph - (p.kh - 1) * p.dh, ow0 = w + p.pw - (p.kw - 1) * p.dw, ow = ow0, j = p.kw;
+      for (int tap = 0; tap < taps; ++tap, ++it) {
+        const uint32_t buf = it % kBufs, bph = (it / kBufs) & 1u;
+        const bool reached = (unsigned)oh < (unsigned)p.OH && (unsigned)ow < (unsigned)p.OW;
+        const float ta = reached ? sa : 0.0f, tb = reached ? fb : 0.0f;
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait_parked(&tmem_full[buf], bph, abort_flag, p.wait_ns)) != 0;
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < kChunks; ++k)
+          if (k < mine) {  // (the same in every lane of the warp)
+            uint32_t acc[32];
+            __syncwarp();
+            tmem_ld32(tmem_base + buf * L::kMaxBN + ((uint32_t)(q * 32) << 16) + (first + k) * 32, acc);
+            if (ONE) open(sum[0]);
+            add(sum[ONE ? 0 : k], acc, ta, tb);
+            if (ONE && inside) store(sum[0], first + k);
+          }
+        tc_fence_before();
+        __syncwarp();
+        if (elect_one()) mbar_arrive(&tmem_empty[buf]);
+        ow += p.dw;
+        if (--j == 0) {
+          j = p.kw;
+          ow = ow0;
+          oh += p.dh;
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (elect_one()) mbar_arrive(&tmem_empty[buf]);
+      if (!ONE && ok && inside) {
+#pragma unroll
+        for (int k = 0; k < kSums; ++k)
+          if (k < mine) store(sum[k], first + k);
+      }
     }
   }
 
@@ -218,8 +277,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 }  // namespace
 
-// Whether conv_grad_input makes the input gradient: stride 1, one scale for the codes of an image, one byte per code, sums that 32 bits
-// hold.  (A dilation wider than the output leaves positions that no tap reaches, which have to be 0 whatever the scales.)
+// Whether conv_grad_input makes the input gradient: stride 1, one scale for the codes of an image, one byte per code, sums of a tap that 32
+// bits hold.  (Under a dilation wider than the output most taps reach nothing.)
 bool conv_fold_covered(const hot_layer_t& l, const hot_conv_t& v) {
   const hot_linear_cfg_t& c = l.cfg;
   if (v.B <= 0 || v.C <= 0 || v.H <= 0 || v.W <= 0 || v.kh <= 0 || v.kw <= 0 || v.dh <= 0 || v.dw <= 0 || v.ph < 0 || v.pw < 0 || v.dtype != c.dtype ||
@@ -228,8 +287,7 @@ bool conv_fold_covered(const hot_layer_t& l, const hot_conv_t& v) {
   if (v.sh != 1 || v.sw != 1 || c.q_gx.scale_mode != HOT_SCALE_TENSOR || c.q_gx.storage != HOT_STORE_INT8) return false;
   const int64_t oh = v.H + 2 * v.ph - (int64_t)v.dh * (v.kh - 1), ow = v.W + 2 * v.pw - (int64_t)v.dw * (v.kw - 1);
   if (oh < v.dh || ow < v.dw || oh > (1 << 20) || ow > (1 << 20) || v.H > (1 << 20) || v.W > (1 << 20) || v.C > (1 << 20) || v.B > 65535) return false;
-  const int64_t k = l.O * (int64_t)v.kh * v.kw;
-  return k * 128 * ((1ll << (c.q_w.bits - 1)) - 1) < (1ll << 31) && v.kh * (int64_t)v.kw <= 4096 && l.I == (int64_t)v.C * v.kh * v.kw &&
+  return l.O * 128 * ((1ll << (c.q_w.bits - 1)) - 1) < (1ll << 31) && v.kh * (int64_t)v.kw <= 4096 && l.I == (int64_t)v.C * v.kh * v.kw &&
          (l.batch ? l.batch == v.B && l.L == oh * ow : l.L == v.B * oh * ow);
 }
 
@@ -251,14 +309,15 @@ int conv_grad_input(const hot_layer_t& l, const hot_conv_t& v, const void* q_go,
   p.th = (p.H + rows - 1) / rows;
   p.bh = (p.H + p.th - 1) / p.th;
   p.tw = (p.W + p.bw - 1) / p.bw;
-  // channels: up to 256, fewer where that leaves SMs idle
+  // channels: as many as fit, fewer where that leaves SMs idle
   const int64_t m_tiles = (int64_t)v.B * p.th * p.tw;
-  p.bn = p.C >= kMaxBN ? kMaxBN : (p.C + 31) / 32 * 32;
+  const int most = taps == 1 ? Layout<true>::kMaxBN : Layout<false>::kMaxBN;
+  p.bn = p.C >= most ? most : (p.C + 31) / 32 * 32;
   while (p.bn > 32 && m_tiles * ((p.C + p.bn - 1) / p.bn) < sms) p.bn = (p.bn / 2 + 31) / 32 * 32;
   p.n_tiles = (p.C + p.bn - 1) / p.bn;
   if (m_tiles * p.n_tiles >= (1ll << 30)) HOT_FAIL(HOT_ERR_UNSUPPORTED, "hot_layer_backward_conv: too many tiles");
   p.num_tiles = (int)(m_tiles * p.n_tiles);
-  p.kh = v.kh; p.kw = v.kw; p.dh = v.dh; p.dw = v.dw; p.ph = v.ph; p.pw = v.pw;
+  p.OH = (int)oh; p.OW = (int)ow; p.kh = v.kh; p.kw = v.kw; p.dh = v.dh; p.dw = v.dw; p.ph = v.ph; p.pw = v.pw;
   p.kblocks = (int)((l.O + kBK - 1) / kBK);
   p.last_steps = (int)((l.O - (int64_t)(p.kblocks - 1) * kBK + 31) / 32);
   p.by_n = fast_div(p.n_tiles);
@@ -270,8 +329,9 @@ int conv_grad_input(const hot_layer_t& l, const hot_conv_t& v, const void* q_go,
   p.sa_batch = l.batch > 0;
   p.sb = s_w;
   p.post = post;
+  p.lean = l.I * (l.cfg.dtype == HOT_BF16 ? 2 : 4) % 16 == 0;
+  p.one = 1.0f;
   p.out = out;
-  p.out16 = l.cfg.dtype == HOT_BF16;
   p.status = status;
   p.wait_ns = wait_limit_ns();
   CUtensorMap ma, mb;
@@ -281,26 +341,31 @@ int conv_grad_input(const hot_layer_t& l, const hot_conv_t& v, const void* q_go,
   const int64_t db[3] = {l.O, taps, v.C}, sb[2] = {ld_w, ld_w * taps};
   const int bb[3] = {kBK, 1, p.bn};
   if (int rc = make_map_nd(&mb, q_w, 3, db, sb, bb)) return rc;
-  static PerDeviceOnce once;
-  bool done = false;
-  const int dev = once.current(&done);
-  if (dev < 0) HOT_FAIL(HOT_ERR_CUDA, "hot_layer_backward_conv: cannot query the current CUDA device");
-  if (!done) {
-    HOT_CUDA(cudaFuncSetAttribute(conv_fold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    once.mark(dev);
-  }
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(p.num_tiles < sms ? p.num_tiles : sms));
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = kSmem;
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  HOT_CUDA(cudaLaunchKernelEx(&cfg, conv_fold_kernel, ma, mb, p));
-  return HOT_OK;
+  auto launch = [&](auto kernel, int smem, PerDeviceOnce& once) -> int {
+    bool done = false;
+    const int dev = once.current(&done);
+    if (dev < 0) HOT_FAIL(HOT_ERR_CUDA, "hot_layer_backward_conv: cannot query the current CUDA device");
+    if (!done) {
+      HOT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      once.mark(dev);
+    }
+    cfg.dynamicSmemBytes = smem;
+    HOT_CUDA(cudaLaunchKernelEx(&cfg, kernel, ma, mb, p));
+    return HOT_OK;
+  };
+  static PerDeviceOnce once[4];
+  constexpr int kSmem1 = Layout<true>::kSmem, kSmem = Layout<false>::kSmem;
+  if (l.cfg.dtype == HOT_BF16) return taps == 1 ? launch(conv_fold_kernel<true, true>, kSmem1, once[0]) : launch(conv_fold_kernel<false, true>, kSmem, once[1]);
+  return taps == 1 ? launch(conv_fold_kernel<true, false>, kSmem1, once[2]) : launch(conv_fold_kernel<false, false>, kSmem, once[3]);
 }
 
 }  // namespace hot
