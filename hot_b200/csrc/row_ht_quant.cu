@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(kThreads, kPairs == 1 ? 3 : 1) row_ht_quant_ro
         const bool ok1 = ri + 1 < nrun;
         uint32_t w[2][4];
         const uint64_t e0 = (uint64_t)row * (uint64_t)cols + (uint64_t)ri * 16u;
-      quantise32<ROUND, STORE4, false>(v[j], sp, q, e0, true, ok1, w);
+        quantise32<ROUND, STORE4, false>(v[j], sp, q, e0, true, ok1, w);
         uint8_t* dst = cr + (int64_t)ri * (STORE4 ? 8 : 16);
         if (STORE4 && ok1 && ((uintptr_t)dst & 15) == 0) {
           *reinterpret_cast<uint4*>(dst) = make_uint4(w[0][0], w[0][1], w[1][0], w[1][1]);
@@ -420,16 +420,28 @@ struct Stream {
   static constexpr int kBytes = kThreads / 32 * kStages * WarpTile<T>::kBytes;
 };
 
-// The streamed tensor; contig: pitch == cols, so that it is one flat sequence of runs and no division is needed.
+// The streamed tensor, row-major over rows x nrun runs; contig, contig_q: the rows of x, of the codes, follow one another without a gap,
+// so that no division is needed.
 struct Runs {
   int64_t total, ldx, ld_codes;
   int nrun;
-  bool contig, wide;  // wide: runs start on 32-byte boundaries
-  // where run `item` (row-major over rows x nrun) lies, for rows of `ld` elements and runs of `size`
-  __device__ __forceinline__ int64_t at(int64_t item, int64_t ld, int size) const {
-    if (contig) return item * size;
-    const int64_t row = (uint64_t)item >> 32 ? item / nrun : (int64_t)((uint32_t)item / (uint32_t)nrun);
-    return row * ld + (item - row * nrun) * size;
+  FastDiv by_nrun;
+  bool contig, contig_q, wide;  // wide: runs start on 32-byte boundaries
+  // A run in the tensor, worked out once for a warp's 64 neighbouring ones.  (With a quotient of its own for every 16-byte piece and
+  // every run of codes, on both sides where only one had gaps, 40000 x 1040 float32 to 4-bit codes took 100.4 us; now 60.8.  In one
+  // launch each with a quotient a pair it had been 74.1.)
+  struct Spot {
+    int64_t row;
+    int run;
+  };
+  __device__ __forceinline__ Spot spot(int64_t item) const {
+    const int64_t row = item >> 31 ? item / nrun : (int64_t)((int)item / by_nrun);
+    return {row, (int)(item - row * nrun)};
+  }
+  // where the run `ahead` (0 .. 63) behind that one begins, for rows of `ld` elements and runs of `size`
+  __device__ __forceinline__ int64_t at(const Spot& s, int ahead, int64_t ld, int size) const {
+    const int run = s.run + ahead, rows = run / by_nrun;
+    return (s.row + rows) * ld + (int64_t)((run - rows * nrun) * size);
   }
 };
 
@@ -437,19 +449,20 @@ struct Runs {
 template <typename T>
 __device__ __forceinline__ void fetch_runs(uint32_t tile, const T* __restrict__ x, int64_t first, const Runs& t, int lane) {
   using W = WarpTile<T>;
+  constexpr int kPerRun = W::kPieces / 2;
   if (t.contig && first >= 0 && first + 64 <= t.total) {
     const char* src = reinterpret_cast<const char*>(x + first * 16) + lane * 16;
 #pragma unroll
     for (int k = 0; k < W::kPieces; ++k)
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(W::to(tile, k, lane)), "l"(src + k * 512) : "memory");
-  } else if (first >= 0) {
-#pragma unroll
+  } else if (first >= 0 && first < t.total) {  // (a loop: unrolled, it costs the streaming loop registers that it spills)
+    const Runs::Spot s = t.spot(first);
+    const int left = (int)(t.total - first < 64 ? t.total - first : 64);
+#pragma unroll 1
     for (int k = 0; k < W::kPieces; ++k) {
-      constexpr int kPerRun = W::kPieces / 2;
-      const int p = k * 32 + lane;
-      const int64_t item = first + p / kPerRun;
-      const bool ok = item < t.total;
-      copy_piece(W::to(tile, k, lane), reinterpret_cast<const char*>(x + (ok ? t.at(item, t.ldx, 16) : 0)) + (ok ? p % kPerRun * 16 : 0), ok);
+      const int p = k * 32 + lane, ahead = p / kPerRun;
+      const bool ok = ahead < left;
+      copy_piece(W::to(tile, k, lane), reinterpret_cast<const char*>(x + (ok ? t.at(s, ahead, t.ldx, 16) : 0)) + (ok ? p % kPerRun * 16 : 0), ok);
     }
   }
   copy_commit();
@@ -475,9 +488,14 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 4 : 3) row_ht_absma
     for (; first < t.total; first += step) {
       const int64_t item = first + 2 * lane;
       const bool ok0 = item < t.total, ok1 = item + 1 < t.total;
-      const T* p0 = x + (ok0 ? t.at(item, t.ldx, 16) : 0);
+      const T *p0 = x + item * 16, *p1 = p0 + 16;
+      if (!t.contig) {
+        const Runs::Spot s = t.spot(first);
+        p0 = x + t.at(s, 2 * lane, t.ldx, 16);
+        p1 = x + t.at(s, 2 * lane + 1, t.ldx, 16);
+      }
       Raw32<T> raw;
-      raw.load(p0, t.contig ? p0 + 16 : x + (ok1 ? t.at(item + 1, t.ldx, 16) : 0), ok0, ok1, t.wide);
+      raw.load(ok0 ? p0 : x, ok1 ? p1 : x, ok0, ok1, t.wide);
       float2 v[16];
       raw.unpack(v);
       butterfly32<N>(v, n, lane);
@@ -529,8 +547,7 @@ __global__ void __launch_bounds__(kThreads, Stream<T>::kCtasPerSm) row_ht_quant_
   wait_for_predecessor();  // (x is no work of the first pass: its copies were under way before)
   const ScalePair sp = scale_from_absmax(__uint_as_float(absmax[blockIdx.y]), q.qmax);
   if (blockIdx.x == 0 && threadIdx.x == 0) scales[blockIdx.y] = sp.s;
-  // whole tiles need no look at where their runs lie, or at the halves of Philox blocks
-  const bool flat = t.contig && (e_base & 31) == 0 && ((uintptr_t)codes & 15) == 0;
+  const bool flat = t.contig_q && (e_base & 31) == 0 && ((uintptr_t)codes & 15) == 0;
   int stage = 0;
   for (; first >= 0; first -= step) {
     fetch_runs(ring + (stage == 0 ? kStages - 1 : stage - 1) * W::kBytes, x, first - (kStages - 1) * step, t, lane);
@@ -543,7 +560,8 @@ __global__ void __launch_bounds__(kThreads, Stream<T>::kCtasPerSm) row_ht_quant_
     __syncwarp();
     butterfly32<N>(v, n, lane);
     uint32_t w[2][4];
-    // logical element index of the pair: row * cols + col == item * 16 in either layout
+    // logical element index of the pair: row * cols + col == item * 16 in either layout; whole tiles need no look at the halves of
+    // Philox blocks, or, in codes without gaps, at where their runs lie
     const uint64_t e0 = e_base + (uint64_t)item * 16u;
     if (flat && first + 64 <= t.total) {
       quantise32<ROUND, STORE4, true>(v, sp, q, e0, true, true, w);
@@ -556,8 +574,9 @@ __global__ void __launch_bounds__(kThreads, Stream<T>::kCtasPerSm) row_ht_quant_
       }
     } else {
       quantise32<ROUND, STORE4, false>(v, sp, q, e0, ok0, ok1, w);
-      if (ok0) store_run<STORE4>(codes + t.at(item, t.ld_codes, kRunBytes), w[0]);
-      if (ok1) store_run<STORE4>(codes + t.at(item + 1, t.ld_codes, kRunBytes), w[1]);
+      const Runs::Spot s = t.spot(first);
+      if (ok0) store_run<STORE4>(codes + t.at(s, 2 * lane, t.ld_codes, kRunBytes), w[0]);
+      if (ok1) store_run<STORE4>(codes + t.at(s, 2 * lane + 1, t.ld_codes, kRunBytes), w[1]);
     }
     stage = stage + 1 == kStages ? 0 : stage + 1;
   }
@@ -629,7 +648,7 @@ int launch_typed(const T* x, int64_t rows, int cols, int64_t ldx, int n, const h
       else direct(row_ht_quant_rowscale_kernel<T, ROUND, STORE4, 1, 0>);
     }
   } else {
-    const Runs t = {rows * (cols >> 4), ldx, ld_codes, cols >> 4, ldx == cols && ld_codes == (STORE4 ? cols / 2 : cols),
+    const Runs t = {rows * (cols >> 4), ldx, ld_codes, cols >> 4, fast_div(cols >> 4), ldx == cols, ld_codes == (STORE4 ? cols / 2 : cols),
                     (uintptr_t)x % 32 == 0 && ldx * sizeof(T) % 32 == 0};
     const int sms_per_sample = (sms + batch - 1) / batch;
     const dim3 grid((unsigned)grid_for(t.total, sms_per_sample, Stream<T>::kCtasPerSm), (unsigned)batch);

@@ -641,7 +641,7 @@ def test_row_ht_quant_pairs_of_runs(ops, rows, cols, order, lead, dtype, storage
 
 
 @pytest.mark.parametrize("rows,cols,pad", [(1, 16, 0), (3, 48, 16), (7, 1024, 0), (5, 1040, 0), (600, 1056, 16), (1000, 1536, 0), (9, 8176, 0), (2, 8208, 0),
-                                           (450, 8192, 0), (3000, 96, 16), (4001, 80, 0)])
+                                           (450, 8192, 0), (3000, 96, 16), (4001, 80, 0), (5000, 16, 16)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("storage,bits,rounding", [("int4", 4, "philox"), ("int8", 8, "nearest")])
 @pytest.mark.parametrize("scale", ["tensor", "row"])
