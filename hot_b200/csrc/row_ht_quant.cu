@@ -249,10 +249,12 @@ __device__ __forceinline__ void store_run(uint8_t* dst, const uint32_t (&w)[4]) 
 // ---------------------------------------------------------------------------------------
 // per-row scale: one pass, row resident in registers
 // ---------------------------------------------------------------------------------------
-// Two kernels.  Rows of 4-byte elements come through shared memory, to persistent CTAs; rows of 2-byte elements, and short ones, straight
-// from global memory, a CTA for each row or few: those are bound by issue, and the copies only added to it (us, direct / staged:
-// 16384 x 4096 bf16 47.3 / 47.2, 58932 x 384 22.7 / 25.1, 32768 x 8192 213 / 217; float32 6304 x 3072 22.7 / 20.6, 65536 x 1024
-// 68.7 / 57.5, 12608 x 512 12.0 / 10.4, 10705 x 256 6.3 / 8.3).
+// Two kernels.  Rows straight from global memory, a CTA for each row or few, or, for 4-byte elements alone, through shared memory to
+// persistent CTAs of whole warps per row.  The copies pay where a row fills those warps (up to four lanes of its last may idle) or where
+// the direct kernel's threads, a power of two of them, are more (float32, order 16, 4-bit Philox codes, us, direct and staged: 40000 x 2560
+// 107.1 and 99.5, 1024 columns 33.4 and 33.1, but 528 29.3 and 33.4, 1088 60.0 and 64.1); for codes that take little arithmetic they pay beside
+// the exchanges of order 64 whatever idles (640 columns, nearest, 39.1 and 35.3; 1088 74.5 and 73.5).  Rows of 2-byte elements are bound
+// by issue, and the copies only add to it (16384 x 4096 bf16 47.3 and 47.2, 58932 x 384 22.7 and 25.1, 32768 x 8192 213 and 217).
 //
 // kPairs: pairs of runs per thread (1 or 2).  tpr, the threads of a row: the power of two that gives each one pair, from 4 to
 // the CTA: short rows share a warp.
@@ -609,10 +611,13 @@ int launch_typed(const T* x, int64_t rows, int cols, int64_t ldx, int n, const h
   const QuantDev q = make_quant_dev(hq);
   if (hq.scale_mode == HOT_SCALE_ROW) {
     const int npair = ((cols >> 4) + 1) / 2;
-    const bool staged = sizeof(T) == 4 && npair >= 16;
     int tpr = 4;
-    while (tpr < (staged ? 32 : kThreads) && tpr < npair) tpr <<= 1;  // one pair per thread while a CTA can hold the row
-    if (staged && npair > 32) tpr = npair >= kThreads ? kThreads : (npair + 31) / 32 * 32;
+    while (tpr < kThreads && tpr < npair) tpr <<= 1;  // one pair per thread while a CTA can hold the row
+    const int warps_tpr = npair >= kThreads ? kThreads : (npair + 31) / 32 * 32;
+    // (see above the kernels; rows of more than kThreads pairs are the staged kernel's alone)
+    const bool light = n == 64 && ROUND != HOT_ROUND_STOCH_NOISE && (STORE4 || ROUND == HOT_ROUND_NEAREST);
+    const bool staged = sizeof(T) == 4 && npair > 16 && (warps_tpr < tpr || npair + 4 >= warps_tpr || light);
+    if (staged) tpr = warps_tpr;
     if (npair > kMaxPairs * tpr)
       HOT_FAIL(HOT_ERR_UNSUPPORTED, "hot_row_ht_quant: per-row scale supports cols <= %d (got %d)", kMaxPairs * 32 * kThreads, cols);
     const int rows_per_cta = kThreads / tpr;

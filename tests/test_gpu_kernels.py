@@ -641,7 +641,8 @@ def test_row_ht_quant_pairs_of_runs(ops, rows, cols, order, lead, dtype, storage
 
 
 @pytest.mark.parametrize("rows,cols,pad", [(1, 16, 0), (3, 48, 16), (7, 1024, 0), (5, 1040, 0), (600, 1056, 16), (1000, 1536, 0), (9, 8176, 0), (2, 8208, 0),
-                                           (450, 8192, 0), (3000, 96, 16), (4001, 80, 0), (5000, 16, 16)])
+                                           (450, 8192, 0), (3000, 96, 16), (4001, 80, 0), (5000, 16, 16),
+                                           (300, 928, 0), (300, 2000, 0), (37, 2112, 16)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("storage,bits,rounding", [("int4", 4, "philox"), ("int8", 8, "nearest")])
 @pytest.mark.parametrize("scale", ["tensor", "row"])
@@ -656,6 +657,18 @@ def test_row_ht_quant_through_shared_memory(ops, rows, cols, pad, dtype, storage
     xh = oc.fwht_last(_as_f32(x[:, :cols], dtype), 16)
     u = _noise_for(rounding, (rows, cols), rng, 11, 6)
     ref_c, ref_s = (oc.quant_rows if scale == "row" else oc.quant_tensor)(xh, bits, u)
+    assert np.array_equal(np.atleast_1d(ref_s).astype(np.float32).view(np.uint32), scales.cpu().numpy().view(np.uint32))
+    assert np.array_equal(_codes_from(codes, storage, cols), ref_c)
+
+
+@pytest.mark.parametrize("cols", [512, 576, 1088, 1984])
+@pytest.mark.parametrize("storage,bits,rounding", [("int4", 4, "philox"), ("int4", 3, "nearest"), ("int8", 8, "nearest"), ("int8", 8, "philox")])
+def test_row_ht_quant_rows_of_order_64(ops, cols, storage, bits, rounding):
+    """Float32 rows at order 64 with lanes to spare, on either side of the rule that stages them: bit for bit the oracle's."""
+    rng = np.random.default_rng(cols + bits)
+    x = (rng.standard_normal((301, cols)) * 1e-3).astype(np.float32)
+    codes, scales = ops.row_ht_quant(_dev(x, torch.float32), 64, ops.Quant(bits, storage, rounding, "row", 11, 6))
+    ref_c, ref_s = oc.quant_rows(oc.fwht_last(x, 64), bits, _noise_for(rounding, x.shape, rng, 11, 6))
     assert np.array_equal(np.atleast_1d(ref_s).astype(np.float32).view(np.uint32), scales.cpu().numpy().view(np.uint32))
     assert np.array_equal(_codes_from(codes, storage, cols), ref_c)
 
