@@ -308,6 +308,40 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// What the kernel before this one on the stream wrote, or may have written, read behind griddepcontrol.wait.  A programmatic dependent is on
+// the SMs while that kernel still writes, so the value is not constant for its life, as __ldg or a __restrict__ pointer to const
+// promise: the compiler would be free to load it ahead of the wait.
+__device__ __forceinline__ float load_result(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float2 load_result(const float2* p) {
+  float2 v;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double load_result(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 load_result(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 load_result(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint32_t load_result(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
 // Non-negative floats order like their bit patterns, so an unsigned atomicMax works.
 __device__ __forceinline__ void atomic_absmax(uint32_t* p, float v) { atomicMax(p, __float_as_uint(v)); }
 

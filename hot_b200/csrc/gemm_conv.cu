@@ -175,14 +175,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int per = (p.bn / 32 + kTeams - 1) / kTeams, first = team * per, mine = min(per, p.bn / 32 - first);  // this warp's chunks of 32 channels
     constexpr int kChunks = L::kMaxBN / (32 * kTeams), kSums = ONE ? 1 : kChunks;
     const int64_t plane = (int64_t)p.H * p.W;
-    const float sb = __ldg(p.sb), fb = p.lean ? __fmul_rn(sb, p.post) : sb;
+    const float sb = load_result(p.sb), fb = p.lean ? __fmul_rn(sb, p.post) : sb;
     const float2 post2 = make_float2(p.post, p.post), one2 = make_float2(p.one, p.one);
     uint32_t it = 0;
     bool ok = true;
     for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
       const FoldTile t(p, tile);
       const int h = t.h0 + hh, w = t.w0 + ww;
-      const float sa = __ldg(p.sa + (p.sa_batch ? t.b : 0));
+      const float sa = load_result(p.sa + (p.sa_batch ? t.b : 0));
       const bool inside = hh < p.bh && h < p.H && w < p.W;
       const int64_t at = ((int64_t)t.b * p.C + t.n0) * plane + (int64_t)h * p.W + w;
       float2 sum[kSums][16];

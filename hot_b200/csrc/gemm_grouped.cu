@@ -151,13 +151,13 @@ __global__ void __launch_bounds__(Layout<BN>::kThreads, 1)
       float2 run[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) run[i] = make_float2(-0.0f, -0.0f);  // (-0 + v is v, also for v = -0)
-      float ga = __ldg(sa), gb = __ldg(p.sb);
+      float ga = load_result(sa), gb = load_result(p.sb);
       for (int g = 0; g < p.groups; ++g, ++it) {
         const uint32_t buf = it % kBufs, bph = (it / kBufs) & 1u;
         float ga_next = 0.0f, gb_next = 0.0f;
         if (g + 1 < p.groups) {  // in flight during the wait
-          ga_next = __ldg(sa + (g + 1) * sa_step);
-          gb_next = __ldg(p.sb + g + 1);
+          ga_next = load_result(sa + (g + 1) * sa_step);
+          gb_next = load_result(p.sb + g + 1);
         }
         ok = __all_sync(0xFFFFFFFFu, mbar_wait_parked(&tmem_full[buf], bph, abort_flag, p.wait_ns)) != 0;
         if (!ok) break;

@@ -585,9 +585,9 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
         for (int i0 = (warp << sub) + (lane >> (5 - sub)); i0 < rows; i0 += 16 * step) {
           float t[16];
 #pragma unroll
-          for (int k = 0; k < 16; ++k) t[k] = i0 + k * step < rows ? __ldg(src + (int64_t)(i0 + k * step) * p.O) : 0.0f;
+          for (int k = 0; k < 16; ++k) t[k] = load_result(src + (int64_t)(i0 + k * step < rows ? i0 + k * step : i0) * p.O);  // (no branches)
 #pragma unroll
-          for (int k = 0; k < 16; ++k) v += t[k];
+          for (int k = 0; k < 16; ++k) v += i0 + k * step < rows ? t[k] : 0.0f;
         }
         if (sub) {
           __syncwarp();

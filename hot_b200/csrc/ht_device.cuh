@@ -6,14 +6,14 @@
 
 namespace hot {
 
-// ---- loads: 16 consecutive elements -> eight (A_i, B_i) pairs ----------------------------
+// ---- loads: 16 consecutive elements -> eight (A_i, B_i) pairs (in kernels that wait for a predecessor) ----
 template <typename T>
 struct Load16;
 template <>
 struct Load16<float> {
   static __device__ __forceinline__ void run(const float* p, float2 (&v)[8]) {
     const float4* q = reinterpret_cast<const float4*>(p);
-    const float4 a0 = __ldg(q), a1 = __ldg(q + 1), b0 = __ldg(q + 2), b1 = __ldg(q + 3);
+    const float4 a0 = load_result(q), a1 = load_result(q + 1), b0 = load_result(q + 2), b1 = load_result(q + 3);
     v[0] = make_float2(a0.x, b0.x); v[1] = make_float2(a0.y, b0.y);
     v[2] = make_float2(a0.z, b0.z); v[3] = make_float2(a0.w, b0.w);
     v[4] = make_float2(a1.x, b1.x); v[5] = make_float2(a1.y, b1.y);
@@ -24,7 +24,7 @@ template <>
 struct Load16<__nv_bfloat16> {
   static __device__ __forceinline__ void run(const __nv_bfloat16* p, float2 (&v)[8]) {
     const uint4* q = reinterpret_cast<const uint4*>(p);
-    const uint4 a = __ldg(q), b = __ldg(q + 1);
+    const uint4 a = load_result(q), b = load_result(q + 1);
     const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {

@@ -92,12 +92,12 @@ template <typename T>
 struct Pair;
 template <>
 struct Pair<float> {
-  static __device__ __forceinline__ float2 load(const char* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
+  static __device__ __forceinline__ float2 load(const char* p) { return load_result(reinterpret_cast<const float2*>(p)); }
 };
 template <>
 struct Pair<__nv_bfloat16> {
   static __device__ __forceinline__ float2 load(const char* p) {
-    const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(p));
+    const uint32_t w = load_result(reinterpret_cast<const uint32_t*>(p));
     return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
   }
 };
@@ -131,7 +131,7 @@ __device__ __forceinline__ float warp_max_abs(float v) { return __uint_as_float(
 // maximum of n non-negative partials, the same in every lane of every warp
 __device__ __forceinline__ float max_of_partials(const float* p, int n) {
   float m = 0.0f;
-  for (int i = threadIdx.x & 31; i < n; i += 32) m = fmaxf(m, __ldg(p + i));
+  for (int i = threadIdx.x & 31; i < n; i += 32) m = fmaxf(m, load_result(p + i));
   return warp_max_abs(m);
 }
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0); }  // warp-uniform
@@ -155,7 +155,7 @@ template <>
 struct RawMax<__nv_bfloat16> {  // on packed pairs, re-read from L1
   __nv_bfloat162 m = __nv_bfloat162(__ushort_as_bfloat16(0), __ushort_as_bfloat16(0));
   __device__ __forceinline__ void add(const float2 (&)[8], const __nv_bfloat16* p) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(p)), b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+    const uint4 a = load_result(reinterpret_cast<const uint4*>(p)), b = load_result(reinterpret_cast<const uint4*>(p) + 1);
     const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
     for (int i = 0; i < 8; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
@@ -617,7 +617,7 @@ __device__ __forceinline__ void quant_tile(const DevJob& j, int at, uint8_t* sme
       if (ok)
         for (int i = 0; i < j.stiles; ++i) {
           const float* p = j.part_col + ((int64_t)b * j.stiles + i) * j.C + ch;
-          m2 = make_float2(fmaxf(m2.x, __ldg(p)), fmaxf(m2.y, __ldg(p + 1)));
+          m2 = make_float2(fmaxf(m2.x, load_result(p)), fmaxf(m2.y, load_result(p + 1)));
         }
       sa = scale_from_absmax(m2.x, j.qc.qmax);
       sb = scale_from_absmax(m2.y, j.qc.qmax);
@@ -631,8 +631,8 @@ __device__ __forceinline__ void quant_tile(const DevJob& j, int at, uint8_t* sme
       double sq = 0.0, ab = 0.0;
       const double* part = reinterpret_cast<const double*>(j.part_col) + 2 * (int64_t)b * parts;
       for (int i = threadIdx.x; i < parts; i += kThreads) {
-        sq += __ldg(part + 2 * i);
-        ab += __ldg(part + 2 * i + 1);
+        sq += load_result(part + 2 * i);
+        ab += load_result(part + 2 * i + 1);
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
@@ -748,9 +748,11 @@ __device__ __forceinline__ void quant_tile(const DevJob& j, int at, uint8_t* sme
     if (c0 + c < j.C) {
       const float* p = j.part_sum + c0 + c;
       for (int i = q; i < n; i += 8) {
+        float v[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (i + 2 * k < n) s[k] += (double)__ldg(p + (int64_t)(i + 2 * k) * j.C);
+        for (int k = 0; k < 4; ++k) v[k] = load_result(p + (int64_t)(i + 2 * k < n ? i + 2 * k : i) * j.C);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s[k] += i + 2 * k < n ? (double)v[k] : 0.0;
       }
     }
     part[threadIdx.x] = (s[0] + s[1]) + (s[2] + s[3]);
@@ -778,11 +780,12 @@ __device__ __forceinline__ void add_row_sums(const DevJob& j, int block, uint8_t
     for (int i = line; i < n; i += 8 * lines, p += 8 * step) {
       float2 v[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] = i + k * lines < n ? __ldg(reinterpret_cast<const float2*>(p + k * step)) : make_float2(0.0f, 0.0f);
+      for (int k = 0; k < 8; ++k) v[k] = load_result(reinterpret_cast<const float2*>(i + k * lines < n ? p + k * step : p));  // (no branches)
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        s.x += (double)v[k].x;
-        s.y += (double)v[k].y;
+        const bool in = i + k * lines < n;
+        s.x += in ? (double)v[k].x : 0.0;
+        s.y += in ? (double)v[k].y : 0.0;
       }
     }
   }

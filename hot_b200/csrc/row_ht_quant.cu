@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 4 : 3) row_ht_absma
 template <typename T, int ROUND, int STORE4, int N>
 __global__ void __launch_bounds__(kThreads, Stream<T>::kCtasPerSm) row_ht_quant_tensorscale_kernel(
     const T* __restrict__ x, Runs t, int64_t sample, int64_t sample_codes, int n, QuantDev q, uint8_t* __restrict__ codes,
-    float* __restrict__ scales, const uint32_t* __restrict__ absmax) {
+    float* __restrict__ scales, const uint32_t* absmax) {
   // blockIdx.y: sample of a batched call; the Philox / noise element index runs on across samples
   extern __shared__ __align__(16) uint8_t smem[];
   using W = WarpTile<T>;
@@ -547,7 +547,7 @@ __global__ void __launch_bounds__(kThreads, Stream<T>::kCtasPerSm) row_ht_quant_
 #pragma unroll
   for (int k = 0; k < kStages - 1; ++k) fetch_runs(ring + k * W::kBytes, x, first - k * step, t, lane);
   wait_for_predecessor();  // (x is no work of the first pass: its copies were under way before)
-  const ScalePair sp = scale_from_absmax(__uint_as_float(absmax[blockIdx.y]), q.qmax);
+  const ScalePair sp = scale_from_absmax(__uint_as_float(load_result(absmax + blockIdx.y)), q.qmax);
   if (blockIdx.x == 0 && threadIdx.x == 0) scales[blockIdx.y] = sp.s;
   const bool flat = t.contig_q && (e_base & 31) == 0 && ((uintptr_t)codes & 15) == 0;
   int stage = 0;

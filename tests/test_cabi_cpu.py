@@ -151,3 +151,24 @@ def test_which_convolutions_fold_their_own_gradient(cabi, change, covered):
     layer = cabi.HotLayer(change.get("batch", 2), 256, change.get("O", 32), 72, cfg)
     assert lib.hot_conv_folds(ctypes.byref(layer), ctypes.byref(v)) == covered
     assert lib.hot_conv_folds(None, ctypes.byref(v)) == 0
+
+
+def test_results_of_a_programmatic_predecessor_are_not_read_as_constants():
+    """A kernel launched as a programmatic dependent runs while the kernel before it still writes: what that one leaves (maxima, scales,
+    partial sums, the tensor itself) may be read neither by __ldg nor through a __restrict__ pointer to const, which the compiler may load
+    ahead of the wait.  Two files read inputs that way: before their pass of two, which an ordinary launch begins."""
+    csrc = os.path.join(ROOT, "hot_b200", "csrc")
+    inputs = {"row_ht_quant.cu": {"x", "p + k"}, "go_dual_tc.cu": {"src + (int64_t)r * p.ld_wt"}}
+    waiting = []
+    for name in sorted(os.listdir(csrc)):
+        with open(os.path.join(csrc, name)) as f:
+            text = f.read()
+        if "griddepcontrol.wait" not in text or not name.endswith(".cu"):
+            continue
+        waiting.append(name)
+        constant = re.findall(r"__ldg\(([^;]*?)\)(?: << 16\))?;", text) + re.findall(r"const \w+\* __restrict__ (\w+)", text)
+        assert set(constant) <= inputs.get(name, set()), (name, constant)
+        assert text.count("__ldg(") <= len(constant), name
+    assert {"quant_tiles.cu", "gemm_conv.cu", "gemm_grouped.cu", "row_ht_quant.cu", "go_dual.cu", "go_dual_tc.cu", "gemm_i8.cu"} <= set(waiting)
+    with open(os.path.join(csrc, "ht_device.cuh")) as f:
+        assert "__ldg" not in f.read()
