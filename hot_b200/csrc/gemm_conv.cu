@@ -285,8 +285,10 @@ bool conv_fold_covered(const hot_layer_t& l, const hot_conv_t& v) {
       l.O <= 0 || c.q_w.bits < 2 || c.q_w.bits > 8)
     return false;
   if (v.sh != 1 || v.sw != 1 || c.q_gx.scale_mode != HOT_SCALE_TENSOR || c.q_gx.storage != HOT_STORE_INT8) return false;
-  const int64_t oh = v.H + 2 * v.ph - (int64_t)v.dh * (v.kh - 1), ow = v.W + 2 * v.pw - (int64_t)v.dw * (v.kw - 1);
-  if (oh < v.dh || ow < v.dw || oh > (1 << 20) || ow > (1 << 20) || v.H > (1 << 20) || v.W > (1 << 20) || v.C > (1 << 20) || v.B > 65535) return false;
+  const int64_t oh = v.H + 2ll * v.ph - (int64_t)v.dh * (v.kh - 1), ow = v.W + 2ll * v.pw - (int64_t)v.dw * (v.kw - 1);
+  if (oh < v.dh || ow < v.dw || oh > (1 << 20) || ow > (1 << 20) || v.H > (1 << 20) || v.W > (1 << 20) || v.ph > (1 << 20) ||
+      v.pw > (1 << 20) || v.C > (1 << 20) || v.B > 65535)
+    return false;
   return l.O * 128 * ((1ll << (c.q_w.bits - 1)) - 1) < (1ll << 31) && v.kh * (int64_t)v.kw <= 4096 && l.I == (int64_t)v.C * v.kh * v.kw &&
          (l.batch ? l.batch == v.B && l.L == oh * ow : l.L == v.B * oh * ow);
 }
@@ -294,7 +296,7 @@ bool conv_fold_covered(const hot_layer_t& l, const hot_conv_t& v) {
 int conv_grad_input(const hot_layer_t& l, const hot_conv_t& v, const void* q_go, int64_t ld_go, const float* s_go, const void* q_w, int64_t ld_w,
                     const float* s_w, float post, void* out, uint32_t* status, cudaStream_t st) {
   if (!conv_fold_covered(l, v)) HOT_FAIL(HOT_ERR_UNSUPPORTED, "hot_layer_backward_conv: this convolution's input gradient is not folded here");
-  const int64_t oh = v.H + 2 * v.ph - (int64_t)v.dh * (v.kh - 1), ow = v.W + 2 * v.pw - (int64_t)v.dw * (v.kw - 1), taps = (int64_t)v.kh * v.kw;
+  const int64_t oh = v.H + 2ll * v.ph - (int64_t)v.dh * (v.kh - 1), ow = v.W + 2ll * v.pw - (int64_t)v.dw * (v.kw - 1), taps = (int64_t)v.kh * v.kw;
   const int sms = device_sm_count();
   if (sms <= 0) return HOT_ERR_CUDA;
   FoldParams p;

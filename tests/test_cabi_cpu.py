@@ -134,6 +134,7 @@ def test_kept_selection_of_a_matrix_that_comes_to_lie_where_another_did():
 @pytest.mark.parametrize("change,covered", [
     ({}, 1), ({"sh": 2}, 0), ({"sw": 2}, 0), ({"kh": 0}, 0), ({"ph": -1}, 0), ({"dtype": 1}, 0), ({"dh": 40}, 0), ({"H": 15}, 0),
     ({"scale_mode": 1}, 0), ({"storage": 1}, 0), ({"w_bits": 9}, 0), ({"w_bits": 8}, 1), ({"O": 1 << 20, "w_bits": 8}, 0), ({"batch": 3}, 0),
+    ({"H": 20, "ph": 2 ** 31 - 1}, 0), ({"H": 12, "ph": 3}, 1),   # (twice the first padding wraps to -2: 16 rows again)
 ])
 def test_which_convolutions_fold_their_own_gradient(cabi, change, covered):
     """Stride 1, one scale per image, one byte per code, positions that agree with the layer's, every position within reach of a tap, and
