@@ -2,18 +2,22 @@
 //   grad_x[b, c, h, w] = sum over taps (i, j) of round(s_go[b] * s_w * post * sum over o of  q_go[b, h + ph - i dh, w + pw - j dw, o] * q_w[c, (i, j), o])
 //
 // The product over unfolded rows writes kh * kw values per input element, which a fold then reads and adds up.  Here a tile is 128 (or
-// fewer) input positions of one image, whole rows where they fit, by up to 128 channels; for every tap the bulk copy fetches the
+// fewer) input positions, several images where they are small, by up to 128 channels; for every tap the bulk copy fetches the
 // grad_output rows of those positions moved by the tap, with zeros for what lies outside the image, and the kernel's rows of that tap,
 // c * kh * kw + tap, are a dimension of their tensor map.  A tap's integer sums are complete in a tensor-memory buffer of their own; the
 // epilogue scales and rounds them to the tensors' type as the product over rows would and adds them to its registers in the fold's order, so
 // that the result is, bit for bit, what product and fold give (also for scales and gradients that overflow or are infinite): which way a
 // size goes, or whether a layer runs natively, changes no value.  Convolutions of one tap keep no sums and take up to 256 channels.
 //
-// What bounds it: the epilogue (five instructions a value and tap and the conversions; some 600 ns for a tap of 128 x 128), then the fill of
-// shared memory (32 KB per tap and 128 outputs, 250 to 330 ns). 32 x 128 x 28 x 28, 3 x 3, 128 outputs, bf16: the whole training step 159 us, 202
-// with product and fold; sixteen warps in the epilogue, or integers converted by an addition, were 1 to 6 % slower. (Summing the taps
-// as integers, rounded once, takes 154 and gives other values.)
+// What bounds it: the epilogue (five instructions a value and tap and the conversions; some 550 ns for a tap of 128 x 128), then the fill of
+// shared memory (32 KB per tap and 128 outputs, 250 to 330 ns).  The whole training step in bf16, product and fold against this: 32 x 128 x
+// 28 x 28, 3 x 3, to 128 outputs 202 and 156 us; 64 x 512 x 7 x 7, 3 x 3, to 512 169 and 144 (tiles of one image: 155); 256 x 2048 x 4 x 4, 1 x 1,
+// to 512 341 and 317 (one image: 404); 32 x 256 x 56 x 56, 1 x 1, to 64 369 and 308.  Sixteen warps in the epilogue, chunks of 16 channels, or
+// integers converted by an addition were 0 to 6 % slower.  (Summing the taps as integers, rounded once, takes 152 us in the first and
+// gives other values.)
+#include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "layer.cuh"
 #include "tc.cuh"
@@ -28,6 +32,14 @@ constexpr int kBM = 128, kBK = 128;
 constexpr int kEpiWarps = 8, kTeams = kEpiWarps / 4, kThreads = (kEpiWarps + 2) * 32;
 constexpr uint32_t kTmemCols = 512;
 
+// What the choice of a tile, and the choice between this kernel and the product over rows, reckon with (measured): a 128-byte row to shared memory,
+// a tap's channel out of tensor memory, for one tap with its store, what a launch takes besides; the two launches over rows, a byte of
+// theirs written by the product and read by the fold, a CTA of the fold.
+constexpr double kRowNs = 1.05, kDrainNs = 4.7, kDrainOneNs = 3.0, kFoldNs = 4000.0, kRowsNs = 5000.0, kWriteNs = 1 / 3000.0, kReadNs = 1 / 2100.0, kCtaNs = 2.5;
+// The product over rows is taken where this kernel would take clearly longer: few tiles of many outputs, whose k-blocks follow one another (the whole
+// step of 16 x 64 x 14 x 14, 3 x 3, to 1024, bf16: 83.5 us, 75.6 by product and fold; 1 x 512 x 7 x 7 to 512 51.4 and 47.8).
+constexpr double kFoldOver = 1.25;
+
 // ONE: convolutions of one tap
 template <bool ONE>
 struct Layout {
@@ -39,13 +51,13 @@ struct Layout {
 };
 
 struct FoldParams {
-  int H, W, C;
-  int bw, bh;               // positions of a tile: bw columns of bh rows
+  int B, H, W, C;
+  int bw, bh, nb;           // positions of a tile: bw columns of bh rows of nb images
   int tw, th;               // tiles across an image, and down
   int n_tiles, num_tiles, bn;
   int OH, OW, kh, kw, dh, dw, ph, pw;
   int kblocks, last_steps;  // k-blocks of a tap; instructions of 32 in the last of them
-  FastDiv by_n, by_tw, by_th, by_bw;
+  FastDiv by_n, by_tw, by_th, by_bw, by_image;  // (by_image: positions of a tile in one image)
   uint32_t tx;              // bytes of a stage
   const float* sa;
   int sa_batch;             // one scale per image
@@ -73,10 +85,11 @@ struct FoldTile {
   int b, h0, w0, n0;
   __device__ __forceinline__ FoldTile(const FoldParams& p, int tile) {
     const int m = tile / p.by_n, row = m / p.by_tw;
-    b = row / p.by_th;
+    const int images = row / p.by_th;
+    b = images * p.nb;
     n0 = (tile - m * p.n_tiles) * p.bn;
     w0 = (m - row * p.tw) * p.bw;
-    h0 = (row - b * p.th) * p.bh;
+    h0 = (row - images * p.th) * p.bh;
   }
 };
 
@@ -171,7 +184,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else {
     const int q = warp & 3, team = warp >> 2;  // tensor-memory lane quarter; share of the tile's columns
-    const int m = q * 32 + lane, hh = m / p.by_bw, ww = m - hh * p.bw;
+    const int m = q * 32 + lane, image = m / p.by_image, pos = m - image * (p.bw * p.bh), hh = pos / p.by_bw, ww = pos - hh * p.bw;
     const int per = (p.bn / 32 + kTeams - 1) / kTeams, first = team * per, mine = min(per, p.bn / 32 - first);  // this warp's chunks of 32 channels
     constexpr int kChunks = L::kMaxBN / (32 * kTeams), kSums = ONE ? 1 : kChunks;
     const int64_t plane = (int64_t)p.H * p.W;
@@ -181,10 +194,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     bool ok = true;
     for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
       const FoldTile t(p, tile);
-      const int h = t.h0 + hh, w = t.w0 + ww;
-      const float sa = load_result(p.sa + (p.sa_batch ? t.b : 0));
-      const bool inside = hh < p.bh && h < p.H && w < p.W;
-      const int64_t at = ((int64_t)t.b * p.C + t.n0) * plane + (int64_t)h * p.W + w;
+      const int b = t.b + image, h = t.h0 + hh, w = t.w0 + ww;
+      const bool inside = image < p.nb && b < p.B && h < p.H && w < p.W;
+      const float sa = load_result(p.sa + (p.sa_batch && inside ? b : 0));
+      const int64_t at = ((int64_t)b * p.C + t.n0) * plane + (int64_t)h * p.W + w;
       float2 sum[kSums][16];
       auto open = [&](float2 (&v)[16]) {
 #pragma unroll
@@ -192,12 +205,12 @@ __global__ void __launch_bounds__(kThreads, 1)
       };
       // one tap of 32 channels: scaled and rounded as the product over rows stores it, then added.  (A tap outside the output has sums of
       // zero and comes with scales of zero: it adds nothing.)
-      auto add = [&](float2 (&v)[16], const uint32_t (&acc)[32], float ta, float tb) {
+      auto add = [&](auto lean, float2 (&v)[16], const uint32_t (&acc)[32], float ta, float tb) {
         const float2 fa2 = make_float2(ta, ta), fb2 = make_float2(tb, tb);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           float2 f = __fmul2_rn(__fmul2_rn(make_float2((float)(int)acc[2 * i], (float)(int)acc[2 * i + 1]), fa2), fb2);
-          if (!p.lean) f = __fmul2_rn(f, post2);
+          if (!decltype(lean)::value) f = __fmul2_rn(f, post2);
           if (OUT16) {
             const __nv_bfloat162 r = __floats2bfloat162_rn(f.x, f.y);
             const uint32_t bits = *reinterpret_cast<const uint32_t*>(&r);
@@ -221,6 +234,23 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (i < left) *o = i & 1 ? v[i / 2].y : v[i / 2].x;
         }
       };
+      // the sum of one tap in 16 bits: rounded, and 0 in place of -0
+      auto store_one = [&](const uint32_t (&acc)[32], float ta, float tb, int c) {
+        const int left = p.C - t.n0 - c * 32;
+        const float2 fa2 = make_float2(ta, ta), fb2 = make_float2(tb, tb);
+        const __nv_bfloat162 zero = __nv_bfloat162(__ushort_as_bfloat16(0), __ushort_as_bfloat16(0));
+        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + at + (int64_t)(c * 32) * plane;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          float2 f = __fmul2_rn(__fmul2_rn(make_float2((float)(int)acc[2 * i], (float)(int)acc[2 * i + 1]), fa2), fb2);
+          if (!p.lean) f = __fmul2_rn(f, post2);
+          const __nv_bfloat162 r = __hadd2_rn(__floats2bfloat162_rn(f.x, f.y), zero);
+          if (2 * i < left) *o = __low2bfloat16(r);
+          o += plane;
+          if (2 * i + 1 < left) *o = __high2bfloat16(r);
+          o += plane;
+        }
+      };
       if (!ONE)
 #pragma unroll
         for (int k = 0; k < kSums; ++k) open(sum[k]);
@@ -238,8 +268,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             uint32_t acc[32];
             __syncwarp();
             tmem_ld32(tmem_base + buf * L::kMaxBN + ((uint32_t)(q * 32) << 16) + (first + k) * 32, acc);
+            if (ONE && OUT16) {
+              if (inside) store_one(acc, ta, tb, first + k);
+              continue;
+            }
             if (ONE) open(sum[0]);
-            add(sum[ONE ? 0 : k], acc, ta, tb);
+            if (p.lean) add(std::true_type(), sum[ONE ? 0 : k], acc, ta, tb);
+            else add(std::false_type(), sum[ONE ? 0 : k], acc, ta, tb);
             if (ONE && inside) store(sum[0], first + k);
           }
         tc_fence_before();
@@ -275,6 +310,58 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
+// How the positions and channels are cut into tiles, and how long that takes.
+struct FoldPlan {
+  int bw, bh, nb, tw, th, bn, n_tiles;
+  int64_t m_tiles;
+  double ns;
+};
+
+// A tile: several whole images where 128 positions hold them, else what needs fewest tiles of an image among whole rows and rows in up to
+// eight more stretches than they must be cut into, evened out over the image and the batch.  Channels: what takes the busiest SM least.
+FoldPlan plan_fold(const hot_layer_t& l, const hot_conv_t& v, int sms) {
+  FoldPlan f = {};
+  const int taps = v.kh * v.kw, kblocks = (int)((l.O + kBK - 1) / kBK);
+  int64_t image_tiles = 0;
+  for (int cut = (v.W + kBM - 1) / kBM, last = cut + 8; cut <= last && cut <= v.W; ++cut) {
+    const int bw = (v.W + cut - 1) / cut, tw = (v.W + bw - 1) / bw, rows = kBM / bw < v.H ? kBM / bw : v.H, th = (v.H + rows - 1) / rows;
+    if (image_tiles && (int64_t)tw * th >= image_tiles) continue;
+    image_tiles = (int64_t)tw * th;
+    f.bw = bw;
+    f.tw = tw;
+    f.th = th;
+    f.bh = (v.H + th - 1) / th;
+  }
+  f.nb = image_tiles == 1 ? kBM / (v.W * v.H) : 1;
+  if (f.nb > v.B) f.nb = v.B;
+  const int64_t batches = (v.B + f.nb - 1) / f.nb;
+  f.nb = (int)((v.B + batches - 1) / batches);
+  f.m_tiles = batches * image_tiles;
+  const int most = taps == 1 ? Layout<true>::kMaxBN : Layout<false>::kMaxBN;
+  for (int n = (v.C + most - 1) / most, bn_last = 0; bn_last != 32; ++n) {
+    const int bn = ((v.C + n - 1) / n + 31) / 32 * 32, n_tiles = (v.C + bn - 1) / bn;
+    if (bn == bn_last) continue;
+    bn_last = bn;
+    // a tap's copies, or its way out of tensor memory, whichever takes longer; the last one's way out is nobody's cover
+    const double copies = kblocks * (kBM + bn) * kRowNs, drain = bn * (taps == 1 ? kDrainOneNs : kDrainNs);
+    const double ns = (double)((f.m_tiles * n_tiles + sms - 1) / sms) * taps * (copies > drain ? copies : drain) + drain + kFoldNs;
+    if (f.ns && ns >= 0.95 * f.ns) continue;  // (narrower tiles fetch the positions once more each)
+    f.ns = ns;
+    f.bn = bn;
+    f.n_tiles = n_tiles;
+  }
+  return f;
+}
+
+// The same gradient by the product over unfolded rows, tiles of 128 x 256 or the writing of them, and by hot_col2im, which reads them again,
+// an image and a few channels to a CTA.
+double rows_ns(const hot_layer_t& l, const hot_conv_t& v, int sms) {
+  const int taps = v.kh * v.kw, size = v.dtype == HOT_BF16 ? 2 : 4, channels = ((128 / size + taps - 1) / taps + 7) / 8 * 8;
+  const double rows = (double)(l.batch ? l.batch * l.L : l.L), bytes = rows * l.I * size;
+  const double rounds = ceil(ceil(rows / 128) * ceil(l.I / 256.0) / sms), product = rounds * ((l.O + kBK - 1) / kBK) * (128 + 256) * kRowNs;
+  return kRowsNs + (product > bytes * kWriteNs ? product : bytes * kWriteNs) + bytes * kReadNs + v.B * ceil((double)v.C / channels) * kCtaNs;
+}
+
 }  // namespace
 
 // Whether conv_grad_input makes the input gradient: stride 1, one scale for the codes of an image, one byte per code, sums of a tap that 32
@@ -301,24 +388,20 @@ int conv_grad_input(const hot_layer_t& l, const hot_conv_t& v, const void* q_go,
   if (sms <= 0) return HOT_ERR_CUDA;
   FoldParams p;
   memset(&p, 0, sizeof(p));
+  const FoldPlan f = plan_fold(l, v, sms);
+  p.B = (int)v.B;
   p.H = (int)v.H;
   p.W = (int)v.W;
   p.C = (int)v.C;
-  // a tile: as many whole rows as 128 positions hold, evened out over the image, or a stretch of one row
-  p.bw = p.W < kBM ? p.W : kBM;
-  int rows = kBM / p.bw;
-  if (rows > p.H) rows = p.H;
-  p.th = (p.H + rows - 1) / rows;
-  p.bh = (p.H + p.th - 1) / p.th;
-  p.tw = (p.W + p.bw - 1) / p.bw;
-  // channels: as many as fit, fewer where that leaves SMs idle
-  const int64_t m_tiles = (int64_t)v.B * p.th * p.tw;
-  const int most = taps == 1 ? Layout<true>::kMaxBN : Layout<false>::kMaxBN;
-  p.bn = p.C >= most ? most : (p.C + 31) / 32 * 32;
-  while (p.bn > 32 && m_tiles * ((p.C + p.bn - 1) / p.bn) < sms) p.bn = (p.bn / 2 + 31) / 32 * 32;
-  p.n_tiles = (p.C + p.bn - 1) / p.bn;
-  if (m_tiles * p.n_tiles >= (1ll << 30)) HOT_FAIL(HOT_ERR_UNSUPPORTED, "hot_layer_backward_conv: too many tiles");
-  p.num_tiles = (int)(m_tiles * p.n_tiles);
+  p.bw = f.bw;
+  p.bh = f.bh;
+  p.nb = f.nb;
+  p.tw = f.tw;
+  p.th = f.th;
+  p.bn = f.bn;
+  p.n_tiles = f.n_tiles;
+  if (f.m_tiles * p.n_tiles >= (1ll << 30)) HOT_FAIL(HOT_ERR_UNSUPPORTED, "hot_layer_backward_conv: too many tiles");
+  p.num_tiles = (int)(f.m_tiles * p.n_tiles);
   p.OH = (int)oh; p.OW = (int)ow; p.kh = v.kh; p.kw = v.kw; p.dh = v.dh; p.dw = v.dw; p.ph = v.ph; p.pw = v.pw;
   p.kblocks = (int)((l.O + kBK - 1) / kBK);
   p.last_steps = (int)((l.O - (int64_t)(p.kblocks - 1) * kBK + 31) / 32);
@@ -326,7 +409,8 @@ int conv_grad_input(const hot_layer_t& l, const hot_conv_t& v, const void* q_go,
   p.by_tw = fast_div(p.tw);
   p.by_th = fast_div(p.th);
   p.by_bw = fast_div(p.bw);
-  p.tx = (uint32_t)((p.bw * p.bh + p.bn) * kBK);
+  p.by_image = fast_div(p.bw * p.bh);
+  p.tx = (uint32_t)((p.bw * p.bh * p.nb + p.bn) * kBK);
   p.sa = s_go;
   p.sa_batch = l.batch > 0;
   p.sb = s_w;
@@ -338,7 +422,7 @@ int conv_grad_input(const hot_layer_t& l, const hot_conv_t& v, const void* q_go,
   p.wait_ns = wait_limit_ns();
   CUtensorMap ma, mb;
   const int64_t da[4] = {l.O, ow, oh, v.B}, sa[3] = {ld_go, ld_go * ow, ld_go * ow * oh};
-  const int ba[4] = {kBK, p.bw, p.bh, 1};
+  const int ba[4] = {kBK, p.bw, p.bh, p.nb};
   if (int rc = make_map_nd(&ma, q_go, 4, da, sa, ba)) return rc;
   const int64_t db[3] = {l.O, taps, v.C}, sb[2] = {ld_w, ld_w * taps};
   const int bb[3] = {kBK, 1, p.bn};
@@ -373,5 +457,9 @@ int conv_grad_input(const hot_layer_t& l, const hot_conv_t& v, const void* q_go,
 }  // namespace hot
 
 extern "C" int hot_conv_folds(const hot_layer_t* layer, const hot_conv_t* conv) {
-  return layer && conv && hot::conv_fold_covered(*layer, *conv) ? 1 : 0;
+  using namespace hot;
+  if (!layer || !conv || !conv_fold_covered(*layer, *conv)) return 0;
+  int sms = device_sm_count();
+  if (sms <= 0) sms = 148;  // (asked where there is no device)
+  return plan_fold(*layer, *conv, sms).ns <= kFoldOver * rows_ns(*layer, *conv, sms) ? 1 : 0;
 }

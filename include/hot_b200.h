@@ -416,8 +416,9 @@ typedef struct hot_conv {
 int hot_im2col(const hot_conv_t* conv, const void* x, void* cols, hot_stream_t stream);
 int hot_col2im(const hot_conv_t* conv, const void* cols, void* x, hot_stream_t stream);
 /* hot_layer_backward of a convolution whose rows are its output positions: grad_x is the input gradient [B, C, H, W] itself, folded by
- * the product that makes it, bit for bit what hot_layer_backward and hot_col2im give.  hot_conv_folds: whether (1 or 0) this layer and convolution are covered (stride 1, one scale per
- * image or for all, one byte per g_x code); where they are not, hot_layer_backward makes the rows and hot_col2im folds them. */
+ * the product that makes it, bit for bit what hot_layer_backward and hot_col2im give.  It covers stride 1, one scale per image or for
+ * all, and one byte per g_x code.  hot_conv_folds: whether (1 or 0) this layer and convolution are covered, and not quicker done by those
+ * two (few positions with many outputs are). */
 int hot_conv_folds(const hot_layer_t* layer, const hot_conv_t* conv);
 int hot_layer_backward_conv(const hot_layer_t* layer, const hot_conv_t* conv, const void* go, const void* w, int64_t ldw, const void* x_q_t,
                             const float* scale_x, void* grad_x, void* grad_w, int64_t ldgw, void* grad_b, void* workspace,

@@ -135,10 +135,11 @@ def test_kept_selection_of_a_matrix_that_comes_to_lie_where_another_did():
     ({}, 1), ({"sh": 2}, 0), ({"sw": 2}, 0), ({"kh": 0}, 0), ({"ph": -1}, 0), ({"dtype": 1}, 0), ({"dh": 40}, 0), ({"H": 15}, 0),
     ({"scale_mode": 1}, 0), ({"storage": 1}, 0), ({"w_bits": 9}, 0), ({"w_bits": 8}, 1), ({"O": 1 << 20, "w_bits": 8}, 0), ({"batch": 3}, 0),
     ({"H": 20, "ph": 2 ** 31 - 1}, 0), ({"H": 12, "ph": 3}, 1),   # (twice the first padding wraps to -2: 16 rows again)
+    ({"O": 4096}, 0),   # (covered: 32 k-blocks a tap on one CTA after another, where the product over rows has them side by side)
 ])
 def test_which_convolutions_fold_their_own_gradient(cabi, change, covered):
-    """Stride 1, one scale per image, one byte per code, positions that agree with the layer's, every position within reach of a tap, and
-    sums that 32 bits hold."""
+    """Stride 1, one scale per image, one byte per code, positions that agree with the layer's, every position within reach of a tap, sums
+    that 32 bits hold, and no product over rows that is the quicker."""
     lib = cabi.lib()
     v = cabi.HotConv(0, 2, 8, 16, 16, 3, 3, 1, 1, 1, 1, 1, 1)
     for k in ("sh", "sw", "kh", "ph", "dtype", "dh", "H"):
