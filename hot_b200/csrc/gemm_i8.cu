@@ -1178,6 +1178,77 @@ double dual_max_load(int64_t t0, int kb0, double ns0, int64_t t1, int kb1, doubl
   }
   return worst;
 }
+// How the two products of a call run.  The decision depends on the shapes and the switches only; a training step asks for the same few again
+// and again, and the replay costs tens of microseconds of host time, so the answers are kept.
+struct DualPlan {
+  int key[14];
+  Plan s0, s1;        // one after the other, or ...
+  bool dual;          // ... in one launch:
+  int bn, split;      // tile width; stretches of k-blocks a rider tile is cut into
+  bool pair, swapped; // on CTA pairs; the main problem is the rider
+};
+
+// One launch pays when the rider's few long tiles fit beside the main problem's last, partly empty wave; otherwise (or with
+// HOT_GEMM_DUAL=0) the two problems run one after the other.  The tile width (HOT_GEMM_DUAL_TILE, else any), and into how many stretches a
+// rider tile is cut (HOT_GEMM_RIDER_SPLIT: 1 leaves them whole), are those whose busiest worker, replayed on the host, has the least to do.
+DualPlan plan_dual(const GemmParams& p0, const GemmParams& p1, bool a4, int sms, const char* together_env, int pair_mode, int force_split, int force_bn,
+                   bool scratch, size_t workspace_bytes) {
+  DualPlan d = {};
+  d.s0 = make_plan(p0.M, p0.N, p0.num_kb, sms, 0, !a4, a4);
+  d.s1 = make_plan(p1.M, p1.N, p1.num_kb, sms, 0, true, false);
+  d.split = 1;
+  double together = 0.0;
+  auto consider = [&](bool swap, bool pair, int bn) {
+    const GemmParams &q0 = swap ? p1 : p0, &q1 = swap ? p0 : p1;
+    const int tile_m = pair ? 2 * kBM : kBM;
+    const int64_t t0 = (int64_t)((q0.M + tile_m - 1) / tile_m) * ((q0.N + bn - 1) / bn);
+    const int64_t t1 = (int64_t)((q1.M + tile_m - 1) / tile_m) * ((q1.N + bn - 1) / bn);
+    const int most = pair ? sms / 2 : sms, workers = (int)(t0 + t1 < most ? t0 + t1 : most);
+    // (every worker holding a rider tile while the lag passes would leave nobody for the main tiles)
+    if (t1 > (pair ? workers - 1 : workers) || (a4 && t0 < workers) || t0 < 1 || t1 < 1) return;
+    // Narrow tiles win only where there are few rounds of them (10705 x 2800 over 256 channels and 10705 tokens, 12 rounds of 128
+    // columns: 38.7 us where the wider plans take 36.9).
+    if (bn < (pair ? 128 : 192) && t0 > 4 * (int64_t)workers && !force_bn) return;
+    const double ns0 = tile_ns(q0.num_kb, bn, pair, a4);
+    for (int split = 1; split <= 4; ++split) {
+      if ((pair || swap) && split > 1) break;  // (the partial sums are parked per worker of one CTA)
+      if (force_split > 0 ? split != force_split : split > 2) continue;  // more than two stretches only when asked (tests)
+      const int piece = (q1.num_kb + split - 1) / split;
+      if (split > 1) {
+        // every stretch non-empty, a slot per worker with a stretch, a counter per rider tile
+        if (!scratch || t0 < workers || t1 * split > sms || (int64_t)(split - 1) * piece >= q1.num_kb || t1 > 160 ||
+            (size_t)(t1 * split) * kBM * bn * sizeof(int32_t) > workspace_bytes)
+          continue;
+      }
+      // Whoever completes a cut tile reads every stretch's sums back from L2, chunk by chunk, and adds them; with the
+      // parking of the sums before it that costs the busiest worker about 10 us for two stretches and more for
+      // three or four (measured at ViT-B sizes: 768 x 768 x 6304 beside 12608 x 768 x 768 gains 2 us from
+      // a cut in two and loses with three or four; larger riders lose with two).
+      const double fix = split > 1 ? 8000.0 + 2300.0 * (split - 2) : 0.0;
+      const double c = launch_ns(bn, pair) + dual_max_load(t0, q0.num_kb, ns0, t1 * split, piece, tile_ns(piece, bn, pair, false), workers) + fix;
+      if (!d.bn || c < together) {
+        d.bn = bn;
+        d.pair = pair;
+        d.split = split;
+        d.swapped = swap;
+        together = c;
+      }
+    }
+  };
+  for (const bool swap : {false, true}) {
+    // Either problem may be the one of few, long tiles: with few tokens it is the first (49 x 768 over 3072 channels, 12 tiles of 24
+    // k-blocks beside 288 of one: 11.6 us in turn, 7.4 in one launch).
+    if (swap && (a4 || force_split > 1 || p0.num_kb <= p1.num_kb)) continue;
+    for (const bool pair : {false, true}) {
+      if (pair ? (pair_mode == 0 || a4 || sms < 2 || force_split > 1) : (pair_mode == 2 && !a4)) continue;
+      for (const int bn : {256, 192, 128, 64})
+        if (!(bn <= 128 && a4) && (!force_bn || bn == force_bn)) consider(swap, pair, bn);
+    }
+  }
+  d.dual = d.bn != 0 && !(together_env && together_env[0] == '0');
+  if (d.dual && !(together_env && together_env[0] == '1')) d.dual = together < d.s0.cost + d.s1.cost;
+  return d;
+}
 }  // namespace
 }  // namespace hot
 
@@ -1196,33 +1267,19 @@ int gemm_i8_dual_ws(const hot_gemm_problem_t* main_problem, const hot_gemm_probl
   const int sms = device_sm_count();
   if (sms <= 0) return HOT_ERR_CUDA;
   const bool a4 = main_problem->a_storage == HOT_STORE_INT4;
-  // One launch pays when the rider's few long tiles fit beside the main problem's last, partly empty
-  // wave; otherwise (or with HOT_GEMM_DUAL=0) the two problems run one after the other.  The tile
-  // width, and into how many stretches of k-blocks a rider tile is cut, are those whose busiest worker,
-  // replayed on the host, has the least to do.
-  const char* env = getenv("HOT_GEMM_DUAL");
-  const char* senv = getenv("HOT_GEMM_RIDER_SPLIT");  // 1: rider tiles stay whole; n: cut into n where possible
-  const int force_split = senv ? atoi(senv) : 0;
-  // The decision depends on the shapes and the switches only; a training step asks for the same few again and
-  // again, and the replay below costs tens of microseconds of host time, so the answers are kept.
-  struct Decision {
-    int key[13];
-    Plan s0, s1;
-    int dual_bn, dual_split;
-    bool dual, dual_pair, swapped;
-  };
+  const char *env = getenv("HOT_GEMM_DUAL"), *senv = getenv("HOT_GEMM_RIDER_SPLIT"), *tenv = getenv("HOT_GEMM_DUAL_TILE");
+  const char *e1 = getenv("HOT_GEMM_SCHEDULE"), *e2 = getenv("HOT_GEMM_PAIR");
+  const int force_split = senv ? atoi(senv) : 0, force_bn = tenv ? atoi(tenv) : 0, pair_mode = e2 ? (e2[0] == '1' ? 2 : (e2[0] == '0' ? 0 : 1)) : 1;
+  const bool scratch = workspace && counters && ((uintptr_t)workspace) % 16 == 0;
   static std::mutex cache_mutex;
-  static std::vector<Decision> cache;
-  const char* e1 = getenv("HOT_GEMM_SCHEDULE");
-  const char* e2 = getenv("HOT_GEMM_PAIR");
-  const bool split_ok = workspace && counters && ((uintptr_t)workspace) % 16 == 0;
-  const int key[13] = {p0.M, p0.N, p0.K, p1.M, p1.N, p1.K, sms, a4 ? 1 : 0, (env ? env[0] : 0) | ((e1 ? e1[0] : 0) << 8) | ((e2 ? e2[0] : 0) << 16),
-                       force_split, split_ok ? 1 : 0, (int)(uint32_t)(workspace_bytes & 0xFFFFFFFFu), (int)(uint32_t)(workspace_bytes >> 32)};
-  Decision dec;
+  static std::vector<DualPlan> cache;
+  const int key[14] = {p0.M, p0.N, p0.K, p1.M, p1.N, p1.K, sms, a4 ? 1 : 0, (env ? env[0] : 0) | ((e1 ? e1[0] : 0) << 8) | ((e2 ? e2[0] : 0) << 16),
+                       force_split, force_bn, scratch ? 1 : 0, (int)(uint32_t)(workspace_bytes & 0xFFFFFFFFu), (int)(uint32_t)(workspace_bytes >> 32)};
+  DualPlan dec;
   bool have = false;
   {
     std::lock_guard<std::mutex> lock(cache_mutex);
-    for (const Decision& d : cache)
+    for (const DualPlan& d : cache)
       if (memcmp(d.key, key, sizeof(key)) == 0) {
         dec = d;
         have = true;
@@ -1230,74 +1287,15 @@ int gemm_i8_dual_ws(const hot_gemm_problem_t* main_problem, const hot_gemm_probl
       }
   }
   if (!have) {
-  const Plan s0 = make_plan(p0.M, p0.N, p0.num_kb, sms, 0, !a4, a4), s1 = make_plan(p1.M, p1.N, p1.num_kb, sms, 0, true, false);
-  int dual_bn = 0, dual_split = 1;
-  bool dual_pair = false, swapped = false;
-  double together = 0.0;
-  const int pair_mode = (e2 ? (e2[0] == '1' ? 2 : (e2[0] == '0' ? 0 : 1)) : 1);
-  for (const bool swap : {false, true})
-  for (const bool pair : {false, true}) {
-    // Either problem may be the one of few, long tiles: with few tokens it is the first (49 x 768 over 3072 channels, 12 tiles of 24
-    // k-blocks beside 288 of one: 11.6 us in turn, 7.4 in one launch).
-    const GemmParams &q0 = swap ? p1 : p0, &q1 = swap ? p0 : p1;
-    if (swap && (a4 || force_split > 1 || q1.num_kb <= q0.num_kb)) continue;
-    if (pair ? (pair_mode == 0 || a4 || sms < 2 || force_split > 1) : (pair_mode == 2 && !a4)) continue;
-    const int tile_m = pair ? 2 * kBM : kBM;
-    for (int bn : {256, 192, 128, 64}) {
-      if (bn <= 128 && a4) continue;
-      const int64_t t0 = (int64_t)((q0.M + tile_m - 1) / tile_m) * ((q0.N + bn - 1) / bn);
-      const int64_t t1 = (int64_t)((q1.M + tile_m - 1) / tile_m) * ((q1.N + bn - 1) / bn);
-      const int most = pair ? sms / 2 : sms, workers = (int)(t0 + t1 < most ? t0 + t1 : most);
-      // (every worker holding a rider tile while the lag passes would leave nobody for the main tiles)
-      if (t1 > (pair ? workers - 1 : workers) || (a4 && t0 < workers) || t0 < 1 || t1 < 1) continue;
-      // Narrow tiles win only where there are few rounds of them (10705 x 2800 over 256 channels and 10705 tokens, 12 rounds of 128
-      // columns: 38.7 us where the wider plans take 36.9).
-      if (bn < (pair ? 128 : 192) && t0 > 4 * (int64_t)workers) continue;
-      const double ns0 = tile_ns(q0.num_kb, bn, pair, a4);
-      for (int split = 1; split <= 4; ++split) {
-        if ((pair || swap) && split > 1) break;  // (the partial sums are parked per worker of one CTA)
-        if (force_split > 0 ? split != force_split : split > 2) continue;  // more than two stretches only when asked (tests)
-        const int piece = (q1.num_kb + split - 1) / split;
-        if (split > 1) {
-          // every stretch non-empty, a slot per worker with a stretch, a counter per rider tile
-          if (!workspace || !counters || t0 < workers || t1 * split > sms || (int64_t)(split - 1) * piece >= q1.num_kb || t1 > 160 ||
-              (size_t)(t1 * split) * kBM * bn * sizeof(int32_t) > workspace_bytes || ((uintptr_t)workspace) % 16 != 0)
-            continue;
-        }
-        // Whoever completes a cut tile reads every stretch's sums back from L2, chunk by chunk, and adds them; with the
-        // parking of the sums before it that costs the busiest worker about 10 us for two stretches and more for
-        // three or four (measured at ViT-B sizes: 768 x 768 x 6304 beside 12608 x 768 x 768 gains 2 us from
-        // a cut in two and loses with three or four; larger riders lose with two).
-        const double fix = split > 1 ? 8000.0 + 2300.0 * (split - 2) : 0.0;
-        const double c = launch_ns(bn, pair) + dual_max_load(t0, q0.num_kb, ns0, t1 * split, piece, tile_ns(piece, bn, pair, false), workers) + fix;
-        if (!dual_bn || c < together) {
-          dual_bn = bn;
-          dual_pair = pair;
-          dual_split = split;
-          swapped = swap;
-          together = c;
-        }
-      }
-    }
-  }
-  bool dual = dual_bn != 0 && !(env && env[0] == '0');
-  if (dual && !(env && env[0] == '1')) dual = together < s0.cost + s1.cost;
+    dec = plan_dual(p0, p1, a4, sms, env, pair_mode, force_split, force_bn, scratch, workspace_bytes);
     memcpy(dec.key, key, sizeof(key));
-    dec.s0 = s0;
-    dec.s1 = s1;
-    dec.dual_bn = dual_bn;
-    dec.dual_split = dual_split;
-    dec.dual_pair = dual_pair;
-    dec.swapped = swapped;
-    dec.dual = dual;
     std::lock_guard<std::mutex> lock(cache_mutex);
     if (cache.size() >= 256) cache.clear();
     cache.push_back(dec);
   }
   const Plan &s0 = dec.s0, &s1 = dec.s1;
-  const int dual_bn = dec.dual_bn, dual_split = dec.dual_split;
-  const bool dual = dec.dual;
-  if (dual) {
+  const int dual_bn = dec.bn, dual_split = dec.split;
+  if (dec.dual) {
     if (dual_split > 1 && clear_words) HOT_CUDA(cudaMemsetAsync(counters, 0, clear_words * sizeof(uint32_t), st));
     const hot_gemm_problem_t *first = dec.swapped ? rider_problem : main_problem, *second = dec.swapped ? main_problem : rider_problem;
     GemmParams &q0 = dec.swapped ? p1 : p0, &q1 = dec.swapped ? p0 : p1;
@@ -1305,10 +1303,10 @@ int gemm_i8_dual_ws(const hot_gemm_problem_t* main_problem, const hot_gemm_probl
     q1.sk_partials = (int32_t*)workspace;
     q1.sk_counters = counters;
     Rider r{second->a, second->lda, second->b, second->ldb, q1};
-    const int tile_m = dec.dual_pair ? 2 * kBM : kBM, most = dec.dual_pair ? sms / 2 : sms;
+    const int tile_m = dec.pair ? 2 * kBM : kBM, most = dec.pair ? sms / 2 : sms;
     auto tiles = [&](const GemmParams& q) { return (int64_t)((q.M + tile_m - 1) / tile_m) * ((q.N + dual_bn - 1) / dual_bn); };
     const int64_t all = tiles(q0) + tiles(q1) * dual_split, workers = all < most ? all : most;
-    const Plan plan{dual_bn, false, (unsigned)(dec.dual_pair ? 2 * workers : workers), dec.dual_pair};
+    const Plan plan{dual_bn, false, (unsigned)(dec.pair ? 2 * workers : workers), dec.pair};
     auto launch = [&](auto packed, auto pair) -> int {
       constexpr bool A4 = decltype(packed)::value, PAIR = decltype(pair)::value;
       switch (dual_bn) {
@@ -1319,7 +1317,7 @@ int gemm_i8_dual_ws(const hot_gemm_problem_t* main_problem, const hot_gemm_probl
       }
     };
     if (a4) return launch(std::true_type(), std::false_type());
-    return dec.dual_pair ? launch(std::false_type(), std::true_type()) : launch(std::false_type(), std::false_type());
+    return dec.pair ? launch(std::false_type(), std::true_type()) : launch(std::false_type(), std::false_type());
   }
   int rc = a4 ? launch_bn<true, false>(main_problem->a, main_problem->lda, main_problem->b, main_problem->ldb, p0, s0, st)
               : launch_bn<false, false>(main_problem->a, main_problem->lda, main_problem->b, main_problem->ldb, p0, s0, st);

@@ -290,11 +290,13 @@ def _run_backward(ops, x, w, go, order_l, sel, dtype, *, gx_row=False, gw_row=Fa
     ((130, 66, 1040), (1040, 66, 65)),           # two row tiles, outputs whose rows are not whole 16-byte pieces
     ((2000, 1024, 1024), (1024, 1024, 1000)),
 ])
-@pytest.mark.parametrize("pair", ["0", "1", None])
-def test_gemm_i8_dual_of_few_tokens(ops, main_shape, rider_shape, pair, monkeypatch):
-    """Either problem may ride, at every tile width and on single CTAs and pairs: bit for bit the separate products."""
+@pytest.mark.parametrize("pair,tile", [("0", "64"), ("0", "128"), ("0", "192"), ("0", "256"), ("1", "128"), ("1", "256"), (None, None)])
+def test_gemm_i8_dual_of_few_tokens(ops, main_shape, rider_shape, pair, tile, monkeypatch):
+    """Whichever problem rides, at every tile width on single CTAs, on pairs and as the planner has it: bit for bit the separate
+    products."""
     if pair:
         monkeypatch.setenv("HOT_GEMM_PAIR", pair)
+        monkeypatch.setenv("HOT_GEMM_DUAL_TILE", tile)
     monkeypatch.setenv("HOT_GEMM_DUAL", "1")
     test_gemm_i8_dual(ops, main_shape, rider_shape, "int8", None, monkeypatch)
 
@@ -562,8 +564,8 @@ def test_weight_quantised_by_the_grad_out_kernels_matches_its_own_kernels(ops, m
     assert torch.equal(out["rides"][1], out["separate"][1])
 
 
-@pytest.mark.parametrize("L,O,I", [(128 * 50, 256, 768), (12608, 768, 768)])
-def test_dual_gemm_with_g_w_tiles_cut_along_the_tokens(ops, monkeypatch, L, O, I):
+@pytest.mark.parametrize("L,O,I,tile", [(128 * 50, 256, 768, None), (12608, 768, 768, None), (128 * 50, 256, 768, "64"), (128 * 50, 256, 768, "128")])
+def test_dual_gemm_with_g_w_tiles_cut_along_the_tokens(ops, monkeypatch, L, O, I, tile):
     """The layer's GEMM launch may cut the few, long tiles of the g_w product into stretches of k-blocks that run on
     different SMs and are summed by whichever finishes last.  Integer sums: the gradients must be bit-identical to
     those of whole tiles, whatever the cut."""
@@ -576,6 +578,8 @@ def test_dual_gemm_with_g_w_tiles_cut_along_the_tokens(ops, monkeypatch, L, O, I
     x_q_t, s_x = ops.abc_compress(x, cfg)
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     monkeypatch.setenv("HOT_GEMM_DUAL", "1")
+    if tile:
+        monkeypatch.setenv("HOT_GEMM_DUAL_TILE", tile)
     out = {}
     for split in ("1", "2", "3", "4"):
         monkeypatch.setenv("HOT_GEMM_RIDER_SPLIT", split)
