@@ -1309,12 +1309,12 @@ int gemm_i8_dual_ws(const hot_gemm_problem_t* main_problem, const hot_gemm_probl
     const Plan plan{dual_bn, false, (unsigned)(dec.pair ? 2 * workers : workers), dec.pair};
     auto launch = [&](auto packed, auto pair) -> int {
       constexpr bool A4 = decltype(packed)::value, PAIR = decltype(pair)::value;
-      switch (dual_bn) {
-        case 256: return launch_gemm<256, A4, false, PAIR>(first->a, first->lda, first->b, first->ldb, q0, plan, st, &r);
-        case 192: return launch_gemm<192, A4, false, PAIR>(first->a, first->lda, first->b, first->ldb, q0, plan, st, &r);
-        case 128: return launch_gemm<128, A4, false, PAIR>(first->a, first->lda, first->b, first->ldb, q0, plan, st, &r);
-        default: return launch_gemm<64, A4, false, PAIR>(first->a, first->lda, first->b, first->ldb, q0, plan, st, &r);
+      if constexpr (!A4) {  // (packed operands take wide tiles only)
+        if (dual_bn == 128) return launch_gemm<128, A4, false, PAIR>(first->a, first->lda, first->b, first->ldb, q0, plan, st, &r);
+        if (dual_bn == 64) return launch_gemm<64, A4, false, PAIR>(first->a, first->lda, first->b, first->ldb, q0, plan, st, &r);
       }
+      return dual_bn == 256 ? launch_gemm<256, A4, false, PAIR>(first->a, first->lda, first->b, first->ldb, q0, plan, st, &r)
+                            : launch_gemm<192, A4, false, PAIR>(first->a, first->lda, first->b, first->ldb, q0, plan, st, &r);
     };
     if (a4) return launch(std::true_type(), std::false_type());
     return dec.pair ? launch(std::false_type(), std::true_type()) : launch(std::false_type(), std::false_type());
