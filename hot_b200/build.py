@@ -22,7 +22,7 @@ LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libhot_b200.so")
 BINDING_PATH = os.path.join(LIB_DIR, "hot_torch.so")
 SOURCES = ["common.cu", "status.cu", "row_ht_quant.cu", "col_ht_quant.cu", "go_dual.cu", "go_dual_tc.cu", "gemm_i8.cu", "linear.cu", "layer.cu",
-           "conv.cu", "quant_tiles.cu", "gemm_grouped.cu", "gemm_conv.cu"]
+           "conv.cu", "quant_tiles.cu", "quant_tiles_f32.cu", "gemm_grouped.cu", "gemm_conv.cu"]
 BINDING_SOURCE = "torch_binding.cpp"
 NVCC_FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
               "-Xcompiler", "-fPIC", "--cudart", "static"]

@@ -817,6 +817,7 @@ __global__ void __launch_bounds__(kThreads, MODE == kColKept || (MODE == kColHal
 }
 
 // ---- host side --------------------------------------------------------------------------------------
+#ifndef HOT_TILES_F32
 bool is_half16(const TileJob& t) {
   if (!t.sel || t.order_col != 16 || t.rank != 8) return false;
   for (int i = 0; i < 8; ++i)
@@ -884,6 +885,8 @@ size_t place_partials(const TileJob& t, const Geometry& g, uint8_t* base, DevJob
   return at;
 }
 
+#endif  // HOT_TILES_F32
+
 template <typename T, int MODE>
 int launch_mode(const DevJobs& jobs, int stats_ctas, int quant_ctas, size_t smem, cudaStream_t st) {
   static PerDeviceOnce once;
@@ -923,6 +926,14 @@ int launch_typed(const DevJobs& jobs, int stats_ctas, int quant_ctas, size_t sme
 }
 
 }  // namespace
+
+// The float32 instances are compiled from this file once more, by quant_tiles_f32.cu: half of what was by far the longest compilation.
+int launch_tiles_f32(const void* jobs, int stats_ctas, int quant_ctas, size_t smem, cudaStream_t st);
+#ifdef HOT_TILES_F32
+int launch_tiles_f32(const void* jobs, int stats_ctas, int quant_ctas, size_t smem, cudaStream_t st) {
+  return launch_typed<float>(*static_cast<const DevJobs*>(jobs), stats_ctas, quant_ctas, smem, st);
+}
+#else
 
 // Whether a job is covered: Philox or nearest rounding, transforms of order up to 16, channel pairs that can be loaded at
 // once, one byte per code on the column side; the row side takes one scale per sample and whole runs of 16 channels.
@@ -1050,8 +1061,9 @@ int launch_tile_jobs(const TileJob* jobs, int count, int dtype, void* scratch, s
     if (t.sum && t.batch * g.stiles > kManyPartials) dev.sums = (int)((t.channels + kSumCh - 1) / kSumCh);
   }
   quant_ctas += dev.sums;
-  if (dtype == HOT_F32) return launch_typed<float>(dev, stats_ctas, quant_ctas, smem, st);
+  if (dtype == HOT_F32) return launch_tiles_f32(&dev, stats_ctas, quant_ctas, smem, st);
   return launch_typed<__nv_bfloat16>(dev, stats_ctas, quant_ctas, smem, st);
 }
+#endif  // HOT_TILES_F32
 
 }  // namespace hot
