@@ -765,7 +765,9 @@ __device__ __forceinline__ void quant_tile(const DevJob& j, int at, uint8_t* sme
 // Row sums of many partials (samples x tiles) come from CTAs of their own (APART): 16 channels each, the partials of every sample and
 // tile in a fixed order, eight loads of a thread in flight.  Summed by the CTAs of the first tiles, half a channel's partials to a thread,
 // they are a tail behind the codes: [32, 784, 128] in bf16, 416 partials, 26.9 us for both launches, 14.2 apart.  Few partials
-// stay there: [64, 197, 2304] and its 64 take 64.7 us, 65.7 apart.
+// stay there: [64, 197, 2304] and its 64 take 64.7 us, 65.7 apart.  Between the two, steps of layers with 100 to 512 partials of 384 to 3072
+// channels are within 1.5 % of one another either way.  (A slice of the channels to each of the first 8 or 16 CTAs, in one kernel: the
+// same layers 0.99 to 1.01, the convolution's step 4 us of 157 slower.)
 constexpr int kManyPartials = 128, kSumCh = 16;
 template <typename T>
 __device__ __forceinline__ void add_row_sums(const DevJob& j, int block, uint8_t* smem) {
@@ -802,10 +804,8 @@ __device__ __forceinline__ void add_row_sums(const DevJob& j, int block, uint8_t
   launch_dependents();
 }
 
-// CTAs per SM: the registers that a loop without spills takes, but for bf16 where six with a few spills are faster (float32,
-// 6304 x 3072 and both other tensors of the extension call: 44.2 us for both launches with six, 42.5 with five).
-// CTAs per SM: the registers that a loop without spills takes where that is faster than six CTAs with a few spills (the extension call's
-// three float32 tensors of 6304 tokens: 44.0 us for both launches with six, 43.4 with five).
+// CTAs per SM: six, whose 80 registers spill some words, but five where kept rows go through shared memory and for float32 with the
+// basis of 8 of 16 (the extension call's three tensors of 6304 tokens: 44.0 us for both launches with six, 43.4 with five).
 template <typename T, int MODE, bool APART>
 __global__ void __launch_bounds__(kThreads, MODE == kColKept || (MODE == kColHalf16 && sizeof(T) == 4) ? 5 : 6) tile_quant_kernel(const __grid_constant__ DevJobs jobs) {
   extern __shared__ __align__(16) uint8_t smem[];  // kept rows as floats [position][64 channels]

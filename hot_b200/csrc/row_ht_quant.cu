@@ -430,8 +430,7 @@ struct Runs {
   FastDiv by_nrun;
   bool contig, contig_q, wide;  // wide: runs start on 32-byte boundaries
   // A run in the tensor, worked out once for a warp's 64 neighbouring ones.  (With a quotient of its own for every 16-byte piece and
-  // every run of codes, on both sides where only one had gaps, 40000 x 1040 float32 to 4-bit codes took 100.4 us; now 60.8.  In one
-  // launch each with a quotient a pair it had been 74.1.)
+  // every run of codes, on both sides where only one had gaps, 40000 x 1040 float32 to 4-bit codes took 100.4 us; now 60.8.)
   struct Spot {
     int64_t row;
     int run;

@@ -275,16 +275,17 @@ struct Saved {
     // the bias gradient comes from the quantisers' own pass over grad_out where they can make it (they take channels in pairs)
     const bool sums = need_b && hot_layer_sums_rows(&l, go.data_ptr()) != 0;
     if (need_b) gb = sums ? at::empty({l.O}, go.options()) : go.reshape({-1, l.O}).sum(0);
-    if (fold)
+    if (fold) {
       check(hot_layer_backward_conv(&l, conv, go.data_ptr(), w2.data_ptr(), w2.stride(0), codes.data_ptr(), (const float*)scale.data_ptr(),
                                     gx.data_ptr(), need_w ? gw.data_ptr() : nullptr, ldgw, sums ? gb.data_ptr() : nullptr, ws.data_ptr(), ws_bytes,
                                     nullptr, current_stream()),
             "hot_layer_backward_conv");
-    else
-    check(hot_layer_backward(&l, go.data_ptr(), w2.data_ptr(), w2.stride(0), codes.data_ptr(), (const float*)scale.data_ptr(),
-                             need_x ? gx.data_ptr() : nullptr, l.I, need_w ? gw.data_ptr() : nullptr, ldgw, sums ? gb.data_ptr() : nullptr,
-                             ws.data_ptr(), ws_bytes, nullptr, current_stream()),
-          "hot_layer_backward");
+    } else {
+      check(hot_layer_backward(&l, go.data_ptr(), w2.data_ptr(), w2.stride(0), codes.data_ptr(), (const float*)scale.data_ptr(),
+                               need_x ? gx.data_ptr() : nullptr, l.I, need_w ? gw.data_ptr() : nullptr, ldgw, sums ? gb.data_ptr() : nullptr,
+                               ws.data_ptr(), ws_bytes, nullptr, current_stream()),
+            "hot_layer_backward");
+    }
     if (need_w && ldgw != l.I) gw = gw.narrow(1, 0, l.I);
   }
 };
